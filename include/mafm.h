@@ -391,7 +391,8 @@ int mafm_df_weights(const mafm_df_params* params, double dz, double* w, int32_t 
 /* df[s][x][y] for every window s of n_w heights (nz - n_w windows, ascending
  * z): fz[((x*ny + y)*nz + k) * stride] is Fz at scan level k (k = 0 at zhigh);
  * stride 8 reads mafm_point.force[2] (pass &pts[0].force[2]).  Host or device
- * memory. */
+ * memory; with device memory on both sides the call is ordered on the stream
+ * and returns without waiting (as mafm_run with device output). */
 int mafm_df(const double* fz, int64_t stride, int32_t nx, int32_t ny, int32_t nz, double dz,
             const mafm_df_params* params, double* df, void* stream);
 /* Transpose of mafm_df: dL/dFz (nx*ny*nz, level order) from dL/ddf. */

@@ -29,6 +29,12 @@ def params(amplitude=AMPLITUDE, k_cantilever=K_CANTILEVER, f0=F0) -> _abi.DfPara
     return _abi.DfParams(amplitude, k_cantilever, f0)
 
 
+def _n_weights(dz: float, prm: _abi.DfParams | None) -> int:
+    n = C.c_int32()
+    check(lib().mafm_df_weights(C.byref(prm) if prm is not None else None, dz, None, 0, C.byref(n), None))
+    return n.value
+
+
 def weights(dz: float, prm: _abi.DfParams | None = None):
     n = C.c_int32()
     fac = C.c_double()
@@ -87,26 +93,37 @@ def _torch_df(fz, dz, prm, adjoint):
                                     C.c_void_p(out.data_ptr()), stream))
     else:
         nz = x.shape[2]
-        nw = len(weights(dz, prm)[0])
+        nw = _n_weights(dz, prm)
         out = torch.empty((max(nz - nw, 0), nx, ny), dtype=torch.float64, device=x.device)
         check(lib().mafm_df(C.c_void_p(x.data_ptr()), 1, nx, ny, nz, dz, pp,
                             C.c_void_p(out.data_ptr()), stream))
     return out
 
 
+_DF_FUNCTION = None   # the autograd function, made at first use (torch is optional here)
+
+
+def _df_function():
+    global _DF_FUNCTION
+    if _DF_FUNCTION is None:
+        import torch
+
+        class _Df(torch.autograd.Function):
+            @staticmethod
+            def forward(ctx, x, dz, prm):
+                ctx.nz = x.shape[2]
+                ctx.dtype = x.dtype
+                ctx.dz, ctx.prm = dz, prm
+                return _torch_df(x, dz, prm, 0).to(x.dtype)
+
+            @staticmethod
+            def backward(ctx, g):
+                return _torch_df(g, ctx.dz, ctx.prm, ctx.nz).to(ctx.dtype), None, None
+
+        _DF_FUNCTION = _Df
+    return _DF_FUNCTION
+
+
 def df_image_torch(fz, dz: float, prm: _abi.DfParams | None = None):
     """Differentiable df images (nshift, nx, ny) of a (nx, ny, nz) Fz tensor."""
-    import torch
-
-    class _Df(torch.autograd.Function):
-        @staticmethod
-        def forward(ctx, x):
-            ctx.nz = x.shape[2]
-            ctx.dtype = x.dtype
-            return _torch_df(x, dz, prm, 0).to(x.dtype)
-
-        @staticmethod
-        def backward(ctx, g):
-            return _torch_df(g, dz, prm, ctx.nz).to(ctx.dtype)
-
-    return _Df.apply(fz)
+    return _df_function().apply(fz, dz, prm)

@@ -127,3 +127,29 @@ def test_df_loss_backpropagates_through_the_relaxation(tmp_path):
     w = odf.df_adjoint(g.cpu().numpy(), desc.c.nz, dz).reshape(-1)
     want = oracle.adjoint(desc, pts, w)["dpos"]
     np.testing.assert_allclose(pos.grad.numpy(), want, rtol=1e-6, atol=1e-9 * np.abs(want).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,nz,dz", [
+    (1, 1, 9, 0.1),          # one column, one window
+    (1, 31, 24, 0.1), (1, 33, 25, 0.1), (3, 11, 40, 0.1),   # around the 32-column tile, even and odd heights
+    (5, 13, 95, 0.1), (4, 9, 191, 0.05), (2, 17, 200, 0.1),  # up to and past the shared-memory tile
+    (2, 3, 300, 0.004)])     # more weights than the kernel argument holds
+def test_df_tiles_match_oracle(nx, ny, nz, dz):
+    torch = pytest.importorskip("torch")
+    fz = _stack(9, nx, ny, nz)
+    want = odf.df_images(fz, dz)
+    g = np.random.default_rng(10).normal(size=want.shape)
+    back = odf.df_adjoint(g, nz, dz)
+    x = torch.tensor(fz, device="cuda", requires_grad=True)
+    img = df.df_image_torch(x, dz)
+    img.backward(torch.tensor(g, device="cuda"))
+    # a window sums at most n terms of FP64: n 2^-53 relative to the largest partial sum
+    n = len(df.weights(dz)[0])
+    w, fac = odf.weights(dz)
+    tol = 4 * n * 2.0 ** -53 * fac * dz * np.abs(w).sum()
+    np.testing.assert_allclose(img.detach().cpu().numpy(), want, rtol=0, atol=tol * np.abs(fz).max())
+    np.testing.assert_allclose(x.grad.cpu().numpy(), back, rtol=0, atol=tol * np.abs(g).max())
+    pts = np.zeros(fz.size, dtype=_abi.POINT_DTYPE)
+    pts["force"][:, 2] = fz.reshape(-1)
+    np.testing.assert_array_equal(df.df_images(pts, dz, shape=fz.shape), img.detach().cpu().numpy())
