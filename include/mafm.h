@@ -171,10 +171,10 @@ typedef struct mafm_run_opts {
                                    (from the column count; mafm_autotune measures).
                                    MAFM_DF: 1,2,4,8 lanes share a column's terms; 0 =
                                    default */
-    int32_t block_threads;      /* 0 = default (256) */
-    int32_t columns_per_tile;   /* FP32C: columns a warp takes from the shared queue at a
+    int32_t block_threads;      /* 0 = default (256; 128 for a batch) */
+    int32_t columns_per_tile;   /* FP32C: columns a warp takes from its scan's queue at a
                                    time; 0 = default (1 for a large single scan, else one
-                                   or four per group) */
+                                   per group) */
     int32_t col_begin;          /* relax only columns [col_begin, col_end) of */
     int32_t col_end;            /*   i*ny + j; 0,0 = all */
 } mafm_run_opts;

@@ -175,7 +175,8 @@ cudaError_t launch_grid_build64(const ScanParams& p, const GridView& g, Node64* 
 struct BatchScan {
     ScanParams p;
     mafm_point* out;          // points of columns [col_begin, col_end), (col-col_begin)*nz+k
-    long long tile_begin;     // first global tile index of this scan
+    float share_begin;        // where the scan's share of the launch's expected work begins, in [0, 1)
+    float weight;             // expected work of one column
     int col_begin, col_end;
     int n_pairs_per_eval;     // vdW + Coulomb terms per force evaluation
     int has_coulomb;
@@ -186,14 +187,18 @@ struct BatchScan {
 struct Relax32Config {
     int lanes;                // lanes per column (1,2,4,8,16,32)
     int block;                // threads per block
-    int cols_per_tile;        // columns per warp work tile
+    int cols_per_tile;        // columns a warp takes from its scan's queue at a time
     int smem_terms;           // terms staged per warp (larger scans read global memory)
     int blocks;               // 0 = fill the GPU
     unsigned long long watchdog_ns;   // persistent-kernel time limit
 };
 
-cudaError_t launch_relax32(const BatchScan* scans_dev, int n_scans, long long n_tiles,
+// n_cols: columns of all scans.  next_col: a queue head per scan, cleared here
+// (may be null for one scan).
+cudaError_t launch_relax32(const BatchScan* scans_dev, int n_scans, long long n_cols, unsigned* next_col,
                            const Relax32Config& cfg, RunCounters* ctr, cudaStream_t s);
+// Fills share_begin and weight of a launch's scans.
+void set_batch_shares(BatchScan* scans, int n_scans);
 // FP64 re-relaxation of listed columns (relax64.cu): list[i] = scan index << 32
 // | column for i < min(count, cap), where count = ctr->n_tie when n_fixed < 0
 // (the columns the double-float kernel flagged) and n_fixed otherwise.

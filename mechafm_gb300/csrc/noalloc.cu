@@ -26,10 +26,14 @@
 namespace mafm {
 namespace {
 
-// Scratch layout: RunCounters at offset 0, the BatchScan list at offset 256.
+// Scratch layout: RunCounters at offset 0, a queue head per scan at offset 64,
+// the BatchScan list at offset 256.
 constexpr size_t kCountersBytes = 256;
+constexpr size_t kQueueOffset = 64;
 constexpr size_t kScratchBytes = kCountersBytes + (size_t)MAFM_NOALLOC_MAX_SCANS * sizeof(BatchScan);
-static_assert(sizeof(RunCounters) <= kCountersBytes, "counters fit their slot");
+static_assert(sizeof(RunCounters) <= kQueueOffset &&
+                  kQueueOffset + MAFM_NOALLOC_MAX_SCANS * sizeof(unsigned) <= kCountersBytes,
+              "counters and queue heads fit their slot");
 
 // Held by every GPU that loads the library until the process exits.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -114,14 +118,14 @@ extern "C" int mafm_run_batch_noalloc(mafm_scan* const* scans, int32_t n_scans,
         unsigned char* base = static_cast<unsigned char*>(scratch_address(device));
         RunCounters* ctr = reinterpret_cast<RunCounters*>(base);
         BatchScan* list = reinterpret_cast<BatchScan*>(base + kCountersBytes);
-        long long tiles = 0;
+        unsigned* next_col = reinterpret_cast<unsigned*>(base + kQueueOffset);
+        std::vector<BatchScan> entries;
+        for (int i = 0; i < n_scans; ++i) entries.push_back(scan_batch_entry(scans[i], outs[i]));
+        set_batch_shares(entries.data(), n_scans);
         DescChunk chunk{};
         int at = 0;
         for (int i = 0; i < n_scans; ++i) {
-            BatchScan b = scan_batch_entry(scans[i], outs[i]);
-            b.tile_begin = tiles;
-            tiles += ((long long)b.col_end + cfg.cols_per_tile - 1) / cfg.cols_per_tile;
-            chunk.b[chunk.n++] = b;
+            chunk.b[chunk.n++] = entries[(size_t)i];
             if (chunk.n == 4 || i == n_scans - 1) {
                 store_descriptors<<<1, 1, 0, st>>>(list + at, chunk);
                 at += chunk.n;
@@ -130,7 +134,7 @@ extern "C" int mafm_run_batch_noalloc(mafm_scan* const* scans, int32_t n_scans,
         }
         cuda_check(cudaGetLastError(), "store descriptors");
         cuda_check(cudaMemsetAsync(ctr, 0, sizeof(RunCounters), st), "clear counters");
-        cuda_check(launch_relax32(list, n_scans, tiles, cfg, ctr, st), "relax32 launch");
+        cuda_check(launch_relax32(list, n_scans, total_cols, next_col, cfg, ctr, st), "relax32 launch");
         // The counters hold the device error word (watchdog, grid exit, staging
         // timeout): read them on every call, so that a failed relaxation is
         // reported whether or not the caller asked for statistics.

@@ -1,12 +1,16 @@
 // relax32.cu — the FP32-compensated GPU path (precision MAFM_FP32C).
 //
-// Persistent, multi-scan relaxation kernel.  Work is a list of tiles of pixel
-// columns, possibly from many scans (a batch); each warp takes one tile at a
-// time with an atomic counter, and G lanes share one column (G = 1..32, a
-// launch parameter from the autotuner or the default rule in scan.cu).  The warp's current scan's
-// tip–atom terms are staged into the warp's slice of shared memory with a
-// bulk copy (cp.async.bulk + mbarrier); every lane of a group sums its share
-// of the terms, then the group combines its sums with xor shuffles.
+// Persistent, multi-scan relaxation kernel.  Every scan of a launch (one, or a
+// batch) has a queue of pixel columns in expected-cost order.  A warp starts
+// with a scan chosen by the scans' shares of the expected work, takes columns
+// from that scan's queue until it is empty, and then moves to the scan with the
+// most expected work left; a move waits for all the warp's columns, so moves
+// are what a batch must not make often.  G lanes share one column (G = 1..32, a
+// launch parameter from the autotuner or the default rule in scan.cu).  The
+// warp's current scan's tip–atom terms are staged into the warp's slice of
+// shared memory with a bulk copy (cp.async.bulk + mbarrier); every lane of a
+// group sums its share of the terms, then the group combines its sums with xor
+// shuffles.
 //
 // The main loop runs in "slots": one force evaluation per group per slot,
 // then a per-group state machine advances FIRE/SD and the integrator
@@ -560,8 +564,12 @@ __device__ __forceinline__ unsigned long long global_ns() {
 
 struct WarpHdr {
     unsigned long long mbar;
-    int assign[32];
-    int pad[2];
+    // the warp's place in its current scan's queue (kept here, not in registers)
+    unsigned t_next, t_end;   // positions taken and not yet started
+    unsigned n_cols;          // columns of the scan
+    int exhausted;            // the queue is empty
+    int cur;                  // the scan, -1 before the first
+    int pad;
     WarpParams wp;
 };
 static_assert(sizeof(WarpHdr) % 16 == 0, "warp header keeps the atom slice 16-byte aligned");
@@ -648,15 +656,14 @@ struct GroupState {
 };
 
 template <int G>
-__global__ void __launch_bounds__(256) relax32_kernel(const BatchScan* __restrict__ scans,
-                                                      int n_scans, long long n_tiles,
-                                                      int cols_per_tile, int smem_terms,
-                                                      unsigned long long watchdog_ns,
-                                                      RunCounters* ctr) {
+__global__ void __launch_bounds__(256, 2) relax32_kernel(const BatchScan* __restrict__ scans,
+                                                         int n_scans, unsigned* next_col,
+                                                         int cols_per_tile, int smem_terms,
+                                                         unsigned long long watchdog_ns,
+                                                         RunCounters* ctr) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int grp = lane / G, lg = lane % G;
-    constexpr int kGroups = 32 / G;
     const size_t slice = sizeof(WarpHdr) + (size_t)smem_terms * sizeof(AtomRec32);
     WarpHdr* hdr = reinterpret_cast<WarpHdr*>(smem_raw + (size_t)warp * slice);
     AtomRec32* sm_terms = reinterpret_cast<AtomRec32*>(hdr + 1);
@@ -665,15 +672,14 @@ __global__ void __launch_bounds__(256) relax32_kernel(const BatchScan* __restric
     if (lane == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&hdr->mbar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        hdr->t_next = hdr->t_end = hdr->n_cols = 0;
+        hdr->exhausted = 1;
+        hdr->cur = -1;
     }
     __syncwarp();
     uint32_t phase = 0;
 
     // warp-uniform state
-    int cur = -1;                 // current scan
-    int t_next = 0, t_end = 0;    // column cursor of the current tile
-    long long pending = -1;       // next tile, of another scan
-    bool exhausted = false;
     const BatchScan* S = nullptr;
     const TermPair32* units = nullptr;
     int n_units = 0, n_units_lj = 0;
@@ -689,14 +695,35 @@ __global__ void __launch_bounds__(256) relax32_kernel(const BatchScan* __restric
     g.col = -1;
     g.ex = g.ey = g.ez = DF{0.f, 0.f};
 
-    auto scan_of_tile = [&](long long t) {
+    // The scan a warp starts with: scan s gets the warps of its share of the
+    // launch's expected work.
+    auto first_scan = [&]() {
+        const float u = ((float)(blockIdx.x * (blockDim.x >> 5) + warp) + 0.5f) /
+                        (float)(gridDim.x * (blockDim.x >> 5));
         int lo = 0, hi = n_scans - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
-            if (scans[mid].tile_begin <= t) lo = mid;
+            if (scans[mid].share_begin <= u) lo = mid;
             else hi = mid - 1;
         }
         return lo;
+    };
+    // The scan with the most expected work left in its queue, -1 for none.
+    auto next_scan = [&]() {
+        float best = 0.f;
+        int at = -1;
+        for (int s = lane; s < n_scans; s += 32) {
+            const unsigned nc = (unsigned)(scans[s].col_end - scans[s].col_begin);
+            const unsigned nx = *reinterpret_cast<volatile unsigned*>(next_col + s);
+            const float left = nx < nc ? (float)(nc - nx) * scans[s].weight : 0.f;
+            if (left > best) { best = left; at = s; }
+        }
+        for (int off = 16; off > 0; off >>= 1) {
+            const float ob = __shfl_xor_sync(kFull, best, off);
+            const int oa = __shfl_xor_sync(kFull, at, off);
+            if (ob > best || (ob == best && oa > at)) { best = ob; at = oa; }
+        }
+        return at;
     };
 
     auto start_level = [&]() {
@@ -746,51 +773,44 @@ __global__ void __launch_bounds__(256) relax32_kernel(const BatchScan* __restric
                 break;
             }
             const unsigned need = __ballot_sync(kFull, lg == 0 && g.col == -1);
-            if (need) {
-                if (lane == 0) {
-                    for (int gi = 0; gi < kGroups; ++gi) {
-                        if (!(need & (1u << (gi * G)))) continue;
-                        int a = -1;
-                        for (;;) {
-                            if (t_next < t_end) { a = t_next++; break; }
-                            if (pending >= 0) { a = -1; break; }
-                            if (exhausted) { a = -2; break; }
-                            const long long t = (long long)atomicAdd(&ctr->next_work, 1ull);
-                            if (t >= n_tiles) { exhausted = true; continue; }
-                            const int s = scan_of_tile(t);
-                            if (s == cur) {
-                                const BatchScan& B = scans[s];
-                                t_next = B.col_begin + (int)(t - B.tile_begin) * cols_per_tile;
-                                t_end = min(B.col_end, t_next + cols_per_tile);
-                                continue;
-                            }
-                            pending = t;
-                        }
-                        hdr->assign[gi] = a;
-                    }
+            if (need && !(hdr->exhausted && hdr->t_next >= hdr->t_end)) {
+                const unsigned wanted = (unsigned)__popc(need);
+                __syncwarp();
+                if (lane == 0 && hdr->t_next >= hdr->t_end) {
+                    const unsigned take = (unsigned)cols_per_tile;   // of the current scan's queue
+                    const unsigned at = atomicAdd(next_col + hdr->cur, take);
+                    hdr->t_next = at;
+                    hdr->t_end = min(hdr->n_cols, at + take);
+                    hdr->exhausted = at + take >= hdr->n_cols;
                 }
                 __syncwarp();
-                t_next = __shfl_sync(kFull, t_next, 0);
-                t_end = __shfl_sync(kFull, t_end, 0);
-                pending = __shfl_sync(kFull, pending, 0);
-                exhausted = __shfl_sync(kFull, (int)exhausted, 0) != 0;
-                if (g.col == -1) {
-                    const int a = hdr->assign[grp];
-                    if (a >= 0) start_column(S->p, S->order ? __ldg(S->order + a) : a);
-                    else if (a == -2) g.col = -2;
-                }
+                const unsigned first = hdr->t_next, end = hdr->t_end;
+                const unsigned a = first + (unsigned)__popc(need & ((1u << (grp * G)) - 1u));
+                if (g.col == -1 && a < end)
+                    start_column(S->p, S->order ? __ldg(S->order + a) : S->col_begin + (int)a);
                 __syncwarp();
+                if (lane == 0) hdr->t_next = max(first, min(end, first + wanted));
+                __syncwarp();
+                if (__any_sync(kFull, g.col == -1)) continue;   // the tile ended: take more, if there is more
             }
             if (__any_sync(kFull, g.col >= 0)) break;
-            if (pending >= 0) {
-                // Every group is idle: switch the warp to the pending tile's scan.
-                const int s = scan_of_tile(pending);
-                cur = s;
+            {
+                // Every group is idle and the queue is empty: another scan.
+                const int s = hdr->cur < 0 ? first_scan() : n_scans > 1 ? next_scan() : -1;
+                if (s < 0) {
+                    alive = false;
+                    break;
+                }
                 S = scans + s;
                 const BatchScan& B = *S;
-                t_next = B.col_begin + (int)(pending - B.tile_begin) * cols_per_tile;
-                t_end = min(B.col_end, t_next + cols_per_tile);
-                pending = -1;
+                __syncwarp();
+                if (lane == 0) {
+                    hdr->cur = s;
+                    hdr->n_cols = (unsigned)(B.col_end - B.col_begin);
+                    hdr->t_next = hdr->t_end = 0;
+                    hdr->exhausted = 0;
+                }
+                __syncwarp();
                 // rigid-grid scans evaluate no direct terms
                 n_units = B.p.n_terms_direct > 0 ? B.p.n_units : 0;
                 n_units_lj = B.p.n_terms_direct > 0 ? B.p.n_units_lj : 0;
@@ -811,12 +831,6 @@ __global__ void __launch_bounds__(256) relax32_kernel(const BatchScan* __restric
                 } else {
                     units = B.p.units32;
                 }
-                if (g.col == -2) g.col = -1;   // groups that found nothing may retry
-                continue;
-            }
-            if (exhausted) {
-                alive = false;
-                break;
             }
         }
         if (!alive) break;
@@ -825,12 +839,12 @@ __global__ void __launch_bounds__(256) relax32_kernel(const BatchScan* __restric
 
         // ---------------- one force evaluation per group ----------------
         Acc acc;
-        acc.zero();
         {
             Tip2 tp;
             tp.hx = f2(g.ex.hi);
             tp.hy = f2(g.ey.hi);
             tp.hz = f2(g.ez.hi);
+            acc.zero();
             if (coul) {
                 sum_units<G, false, true>(units, 0, n_units_lj, lg, tp, acc);
                 sum_units<G, true, true>(units, n_units_lj, n_units, lg, tp, acc);
@@ -1179,7 +1193,7 @@ __global__ void __launch_bounds__(256, 2) grid_build32_kernel(const ScanParams p
 }
 
 template <int G>
-cudaError_t launch_g(const BatchScan* scans, int n_scans, long long n_tiles,
+cudaError_t launch_g(const BatchScan* scans, int n_scans, long long n_cols, unsigned* next_col,
                      const Relax32Config& cfg, RunCounters* ctr, cudaStream_t s) {
     const size_t slice = sizeof(WarpHdr) + (size_t)cfg.smem_terms * sizeof(AtomRec32);
     const size_t smem = slice * (size_t)(cfg.block / 32);
@@ -1194,12 +1208,12 @@ cudaError_t launch_g(const BatchScan* scans, int n_scans, long long n_tiles,
         if (per_sm <= 0) return cudaErrorInvalidConfiguration;
         blocks = sm_count() * per_sm;
     }
-    // No more warps than tiles.
-    const long long warps_needed = n_tiles;
+    // No more warps than full warps of groups (and one more for each scan's rest).
+    const long long warps_needed = (n_cols * G + 31) / 32 + (n_scans > 1 ? n_scans : 0);
     const long long max_blocks = (warps_needed + cfg.block / 32 - 1) / (cfg.block / 32);
     if (blocks > max_blocks) blocks = (int)max_blocks;
     if (blocks < 1) blocks = 1;
-    relax32_kernel<G><<<blocks, cfg.block, smem, s>>>(scans, n_scans, n_tiles, cfg.cols_per_tile,
+    relax32_kernel<G><<<blocks, cfg.block, smem, s>>>(scans, n_scans, next_col, cfg.cols_per_tile,
                                                       cfg.smem_terms, cfg.watchdog_ns, ctr);
     return cudaGetLastError();
 }
@@ -1217,16 +1231,24 @@ int sm_count() {
     return count;
 }
 
-cudaError_t launch_relax32(const BatchScan* scans_dev, int n_scans, long long n_tiles,
+cudaError_t launch_relax32(const BatchScan* scans, int n_scans, long long n_cols, unsigned* next_col,
                            const Relax32Config& cfg, RunCounters* ctr, cudaStream_t s) {
     if (cfg.block % 32 != 0 || cfg.block < 32 || cfg.block > 256) return cudaErrorInvalidValue;
+    if (next_col) {
+        const cudaError_t e = cudaMemsetAsync(next_col, 0, (size_t)n_scans * sizeof(unsigned), s);
+        if (e != cudaSuccess) return e;
+    } else {
+        // one scan: the low word of the counters' own queue head (zeroed with them)
+        if (n_scans != 1) return cudaErrorInvalidValue;
+        next_col = reinterpret_cast<unsigned*>(&ctr->next_work);
+    }
     switch (cfg.lanes) {
-        case 1: return launch_g<1>(scans_dev, n_scans, n_tiles, cfg, ctr, s);
-        case 2: return launch_g<2>(scans_dev, n_scans, n_tiles, cfg, ctr, s);
-        case 4: return launch_g<4>(scans_dev, n_scans, n_tiles, cfg, ctr, s);
-        case 8: return launch_g<8>(scans_dev, n_scans, n_tiles, cfg, ctr, s);
-        case 16: return launch_g<16>(scans_dev, n_scans, n_tiles, cfg, ctr, s);
-        case 32: return launch_g<32>(scans_dev, n_scans, n_tiles, cfg, ctr, s);
+        case 1: return launch_g<1>(scans, n_scans, n_cols, next_col, cfg, ctr, s);
+        case 2: return launch_g<2>(scans, n_scans, n_cols, next_col, cfg, ctr, s);
+        case 4: return launch_g<4>(scans, n_scans, n_cols, next_col, cfg, ctr, s);
+        case 8: return launch_g<8>(scans, n_scans, n_cols, next_col, cfg, ctr, s);
+        case 16: return launch_g<16>(scans, n_scans, n_cols, next_col, cfg, ctr, s);
+        case 32: return launch_g<32>(scans, n_scans, n_cols, next_col, cfg, ctr, s);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -673,7 +673,6 @@ void ensure_order(mafm_scan& s, cudaStream_t st, bool measured = false) {
     BatchScan b{};
     b.p = build_params(s);
     b.out = pts.p;
-    b.tile_begin = 0;
     b.col_begin = 0;
     b.col_end = (int)n;
     b.n_pairs_per_eval = s.n_pairs_per_eval;
@@ -682,9 +681,8 @@ void ensure_order(mafm_scan& s, cudaStream_t st, bool measured = false) {
     write_batch<<<1, 1, 0, st>>>(s.batch.p, b);
     cuda_check(cudaGetLastError(), "descriptor upload");
     const Relax32Config cfg = default_config(n, b.p.n_terms_direct, nullptr, 1);
-    const long long tiles = (n + cfg.cols_per_tile - 1) / cfg.cols_per_tile;
     zero_counters(s, st);
-    cuda_check(launch_relax32(s.batch.p, 1, tiles, cfg, s.ctr.p, st), "cost pilot");
+    cuda_check(launch_relax32(s.batch.p, 1, n, nullptr, cfg, s.ctr.p, st), "cost pilot");
     DevBuf<unsigned> steps;
     steps.alloc((size_t)n);
     column_steps<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(pts.p, s.d.nz, n, steps.p);
@@ -763,25 +761,29 @@ BatchDF batch_df_entry(const mafm_scan& s, mafm_point* out, int cb, int ce, bool
 // when it frees up and the queue (in descending expected cost) stays shared
 // until the last columns; longer tiles reserve columns for a warp's lanes
 // early and leave the end of a launch statically assigned (401 x 401 at G =
-// 1: 100 ms at one column per tile, 114 ms at 32).  Otherwise one column per
-// group: spreading few columns over every warp lowers the active lanes per
-// issued instruction (101 x 101 at G = 2: 43.1 ms at one column per tile,
-// 26.9 ms at 16).  Several scans: four columns per group, because a warp
-// whose next tile belongs to another scan first waits for all its groups:
-// with one-column tiles nearly every warp would wait at every scan boundary
-// (256 scans: 2.3x slower), and longer tiles make those waits rarer (256
-// scans at G = 2: 64-column tiles fastest).
+// 1: 100 ms at one column per tile, 114 ms at 32).  Otherwise, and for several
+// scans, one column per group, so that a warp that starts is a full warp:
+// spreading few columns over every warp lowers the active lanes per issued
+// instruction (201 x 201 at G = 1: 49 ms, 57-66 ms at one column per tile).
+// Several scans: every scan has its own queue and a warp changes scan only
+// when its scan's queue is empty, because a change waits for all its groups.
+// 12 molecules (98,304 columns): 342 ms, at four columns per group 612 ms;
+// with one queue through all scans, where nearly every tile was a change,
+// 669 ms at four and 420 ms at one column per group; 5 small ones (12,801
+// columns) 56 ms against 261 ms.
+// Block: 256 threads; several scans 128, whose warps spread over more SMs when
+// there are few (5 molecules 68 -> 56 ms, 12 molecules the same).
 Relax32Config default_config(long long n_cols, int max_terms, const mafm_run_opts* o, int n_scans) {
     Relax32Config c{};
-    c.block = (o && o->block_threads) ? o->block_threads : 256;
+    c.block = (o && o->block_threads) ? o->block_threads : n_scans > 1 ? 128 : 256;
     const long long lanes_cap = (long long)sm_count() * 512;   // two 256-thread blocks per SM
     int G = 1;
     while (G < 32 && n_cols * G < lanes_cap / 4) G *= 2;
     if (max_terms <= 1) G = 1;
     c.lanes = (o && o->lanes_per_column) ? o->lanes_per_column : G;
     const bool long_queue = n_scans <= 1 && n_cols >= 2 * (lanes_cap / c.lanes);
-    const int tile = n_scans > 1 ? 128 / c.lanes : long_queue ? 1 : 32 / c.lanes;
-    c.cols_per_tile = (o && o->columns_per_tile) ? o->columns_per_tile : tile;
+    const int tile = (o && o->columns_per_tile) ? o->columns_per_tile : long_queue ? 1 : 32 / c.lanes;
+    c.cols_per_tile = std::min(std::max(tile, 1), 1 << 16);   // queue heads are 32-bit
     // Shared slice per warp, in 32 B term slots: the paired records of up to
     // 400 terms (each kind's run padded to even: + 2); 12.9 KB per warp keeps
     // two 8-warp blocks per SM.
@@ -939,8 +941,7 @@ int mafm_run(mafm_scan* scan, const mafm_run_opts* opts, mafm_point* out, mafm_r
             BatchScan b{};
             b.p = build_params(*scan);
             b.out = dout;
-            b.tile_begin = 0;
-            b.col_begin = cb;
+                    b.col_begin = cb;
             b.col_end = ce;
             b.n_pairs_per_eval = scan->n_pairs_per_eval;
             b.has_coulomb = scan->has_coulomb;
@@ -950,8 +951,7 @@ int mafm_run(mafm_scan* scan, const mafm_run_opts* opts, mafm_point* out, mafm_r
             }
             write_batch<<<1, 1, 0, st>>>(scan->batch.p, b);
             const Relax32Config cfg = default_config(ce - cb, b.p.n_terms_direct, opts, 1);
-            const long long n_tiles = ((long long)(ce - cb) + cfg.cols_per_tile - 1) / cfg.cols_per_tile;
-            cuda_check(launch_relax32(scan->batch.p, 1, n_tiles, cfg, scan->ctr.p, st), "relax32 launch");
+            cuda_check(launch_relax32(scan->batch.p, 1, ce - cb, nullptr, cfg, scan->ctr.p, st), "relax32 launch");
         }
         cuda_check(cudaEventRecord(scan->ev1, st), "cudaEventRecord");
         if (staged)
@@ -1012,7 +1012,6 @@ int mafm_run_batch(mafm_scan* const* scans, int32_t n_scans, const mafm_run_opts
             max_terms = std::max(max_terms, s->d.rigidgrid ? 0 : s->P.n_terms);
         }
         Relax32Config cfg = default_config(total_cols, max_terms, opts, n_scans);
-        long long tiles = 0;
         // host outputs: pinned ones are written directly, pageable ones staged
         std::vector<mafm_point*> pinned((size_t)n_scans, nullptr);
         bool any_staged = false;
@@ -1026,20 +1025,21 @@ int mafm_run_batch(mafm_scan* const* scans, int32_t n_scans, const mafm_run_opts
             BatchScan& b = bs[i];
             b.p = build_params_for(*s, dfp);
             b.out = !host_out ? outs[i] : pinned[i] ? pinned[i] : s0->stage.p + offsets[i];
-            b.tile_begin = tiles;
             b.col_begin = 0;
             b.col_end = s->d.nx * s->d.ny;
             b.n_pairs_per_eval = s->n_pairs_per_eval;
             b.has_coulomb = s->has_coulomb;
             b.order = s->order.p;
-            tiles += ((long long)b.col_end + cfg.cols_per_tile - 1) / cfg.cols_per_tile;
         }
+        set_batch_shares(bs.data(), n_scans);
         DevBuf<BatchScan> dbs;
         dbs.alloc(bs.size());
         cuda_check(cudaMemcpyAsync(dbs.p, bs.data(), bs.size() * sizeof(BatchScan), cudaMemcpyHostToDevice, st),
                    "upload batch");
         DevBuf<BatchDF> dbd;
         DevBuf<unsigned long long> rlist;
+        DevBuf<unsigned> next_col;
+        if (!dfp) next_col.alloc((size_t)n_scans);
         if (dfp) {
             std::vector<BatchDF> bd((size_t)n_scans);
             long long first = 0;
@@ -1063,7 +1063,8 @@ int mafm_run_batch(mafm_scan* const* scans, int32_t n_scans, const mafm_run_opts
             cuda_check(launch_repair64(dbs.p, rlist.p, (unsigned)total_cols, -1, true, false, s0->ctr.p, st),
                        "FP64 re-relaxation launch");
         } else {
-            cuda_check(launch_relax32(dbs.p, n_scans, tiles, cfg, s0->ctr.p, st), "relax32 batch launch");
+            cuda_check(launch_relax32(dbs.p, n_scans, total_cols, next_col.p, cfg, s0->ctr.p, st),
+                       "relax32 batch launch");
         }
         cuda_check(cudaEventRecord(s0->ev1, st), "cudaEventRecord");
         if (host_out)
@@ -1242,7 +1243,6 @@ BatchScan scan_batch_entry(const mafm_scan* s, mafm_point* out) {
     BatchScan b{};
     b.p = build_params(*s);
     b.out = out;
-    b.tile_begin = 0;
     b.col_begin = 0;
     b.col_end = s->d.nx * s->d.ny;
     b.n_pairs_per_eval = s->n_pairs_per_eval;
@@ -1257,6 +1257,23 @@ Relax32Config relax32_config(long long n_cols, int max_terms, const mafm_run_opt
 
 void check_run_errors(const RunCounters& c) { check_device_errors(c); }
 
+// Expected work of a column: its term records, and about eight records' worth
+// of minimiser per evaluation (the slot machine is 13 % of a 60-atom
+// cluster's relaxation, 30 records).
+void set_batch_shares(BatchScan* scans, int n_scans) {
+    double total = 0;
+    for (int i = 0; i < n_scans; ++i) {
+        BatchScan& b = scans[i];
+        b.weight = (float)((b.p.n_terms_direct > 0 ? b.p.n_units : 0) + 8);
+        total += (double)b.weight * (b.col_end - b.col_begin);
+    }
+    double sum = 0;
+    for (int i = 0; i < n_scans; ++i) {
+        scans[i].share_begin = total > 0 ? (float)(sum / total) : 0.f;
+        sum += (double)scans[i].weight * (scans[i].col_end - scans[i].col_begin);
+    }
+}
+
 }  // namespace mafm
 
 // ---- batch plans and the autotuner -----------------------------------------
@@ -1264,9 +1281,9 @@ void check_run_errors(const RunCounters& c) { check_device_errors(c); }
 struct mafm_plan {
     int device = 0;
     int n_scans = 0;
-    long long tiles = 0;
     mafm::Relax32Config cfg{};
     mafm::DevBuf<mafm::BatchScan> list;
+    mafm::DevBuf<unsigned> next_col;           // queue head of every scan (FP32C)
     mafm::DevBuf<mafm::RunCounters> ctr;
     // MAFM_DF: the double-float descriptors and the re-relaxation list
     bool dfp = false;
@@ -1283,17 +1300,14 @@ struct mafm_plan {
 namespace mafm {
 namespace {
 
-// Descriptor list of a batch (tile numbering for the persistent kernel).
-std::vector<BatchScan> batch_entries(mafm_scan* const* scans, int n, mafm_point* const* outs,
-                                     const Relax32Config& cfg, long long& tiles, bool df) {
+// Descriptor list of a batch.
+std::vector<BatchScan> batch_entries(mafm_scan* const* scans, int n, mafm_point* const* outs, bool df) {
     std::vector<BatchScan> bs((size_t)n);
-    tiles = 0;
     for (int i = 0; i < n; ++i) {
         bs[i] = scan_batch_entry(scans[i], outs[i]);
         bs[i].p = build_params_for(*scans[i], df);
-        bs[i].tile_begin = tiles;
-        tiles += ((long long)bs[i].col_end + cfg.cols_per_tile - 1) / cfg.cols_per_tile;
     }
+    set_batch_shares(bs.data(), n);
     return bs;
 }
 
@@ -1318,10 +1332,11 @@ void plan_build(mafm_plan& p, mafm_scan* const* scans, int n, const mafm_run_opt
         max_terms = std::max(max_terms, scan_direct_terms(scans[i]));
     }
     p.cfg = default_config(cols, max_terms, opts, n);
-    std::vector<BatchScan> bs = batch_entries(scans, n, outs, p.cfg, p.tiles, p.dfp);
+    std::vector<BatchScan> bs = batch_entries(scans, n, outs, p.dfp);
     p.n_scans = n;
     p.cols = cols;
     p.list.alloc(bs.size());
+    if (!p.dfp) p.next_col.alloc(bs.size());
     p.ctr.alloc(1);
     cuda_check(cudaMemcpyAsync(p.list.p, bs.data(), bs.size() * sizeof(BatchScan),
                                cudaMemcpyHostToDevice, st), "upload plan");
@@ -1351,7 +1366,7 @@ void plan_launch(mafm_plan& p, cudaStream_t st) {
         cuda_check(launch_repair64(p.list.p, p.repair.p, (unsigned)p.cols, -1, true, false, p.ctr.p, st),
                    "FP64 re-relaxation launch");
     } else {
-        cuda_check(launch_relax32(p.list.p, p.n_scans, p.tiles, p.cfg, p.ctr.p, st), "relax32 launch");
+        cuda_check(launch_relax32(p.list.p, p.n_scans, p.cols, p.next_col.p, p.cfg, p.ctr.p, st), "relax32 launch");
     }
 }
 

@@ -209,6 +209,46 @@ def test_no_atoms_and_single_point():
     assert np.abs(got32["tip"] - want["tip"]).max() < 1e-6
 
 
+@pytest.mark.parametrize("lanes,tile,block", [(1, 0, 0), (1, 1, 32), (2, 3, 64), (8, 0, 256), (32, 5, 0),
+                                              (1, 70000, 0), (4, 33, 128)])
+def test_batch_queues_relax_every_column_once(tmp_path, lanes, tile, block):
+    """Scans from one column to several warps, in an order that leaves some
+    without a warp at the start: every point holds the bits of its own run,
+    whatever the shape of the launch, from run_batch, a plan and the
+    allocation-free entry point."""
+    import ctypes as C
+    from mechafm_gb300 import synth
+    torch = pytest.importorskip("torch")
+    sizes = [(1, 1), (40, 33), (1, 2), (7, 9), (31, 1), (3, 11), (1, 1), (16, 16)]
+    scans = []
+    for s, (nx, ny) in enumerate(sizes):
+        spec = synth.molecule_batch(1, seed=s, grids=(8,), atoms=(20, 60), zlow=9.85)[0]
+        spec.options["area"] = f"{0.1 * (nx - 1) + 1e-6!r} {0.1 * (ny - 1) + 1e-6!r}"
+        d = Input(spec.write(str(tmp_path / f"q{s}"))).desc()
+        assert d.shape[:2] == (nx, ny)
+        scans.append(Scan(d, device=0))
+    single = [s.run(_abi.FP32C, lanes=lanes, tile=1)[0] for s in scans]
+    outs, stats = run_batch(scans, lanes=lanes, tile=tile, block=block)
+    assert stats.total_steps == sum(int(p["steps"].sum()) for p in single)
+    for got, want in zip(outs, single):
+        np.testing.assert_array_equal(got, want)
+    bufs = [torch.zeros(s.desc.n_points, 8, dtype=torch.float64, device="cuda") for s in scans]
+    plan = _plan(scans, bufs, _abi.RunOpts(_abi.FP32C, lanes, block, tile, 0, 0))
+    n = len(scans)
+    handles = (C.c_void_p * n)(*[s.handle for s in scans])
+    optrs = (C.c_void_p * n)(*[b.data_ptr() for b in bufs])
+    o = _abi.RunOpts(_abi.FP32C, lanes, block, tile, 0, 0)
+    for launch in (lambda: _abi.lib().mafm_plan_launch(plan, None), lambda: _abi.lib().mafm_plan_launch(plan, None),
+                   lambda: _abi.lib().mafm_run_batch_noalloc(handles, n, C.byref(o), optrs, None, None)):
+        for b in bufs:
+            b.zero_()
+        _abi.check(launch())
+        torch.cuda.synchronize()
+        for b, want in zip(bufs, single):
+            np.testing.assert_array_equal(b.cpu().numpy().view(_abi.POINT_DTYPE).reshape(-1), want)
+    _abi.lib().mafm_plan_destroy(plan)
+
+
 def _plan(scans, outs, opts):
     import ctypes as C
     n = len(scans)
