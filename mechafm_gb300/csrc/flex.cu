@@ -7,18 +7,17 @@
 // integrators then run over all atoms (minimiser.cpp:39-129,
 // integrators.cpp:8-111); convergence looks at the tip only.
 //
-// Layout: one warp per pixel column, the atoms' positions, velocities and
-// force accumulators in the warp's shared-memory slice; lane l owns atoms
-// l, l + 32, ...  The reference sums each atom's force over its interaction
-// list in list order; here every atom has its own list of (interaction kind,
-// index, role) entries in that same order (built on the host), and the lane
-// owning the atom evaluates the entries one after another, so every per-atom
-// sum is formed in the reference's order.  Interactions with several atoms
-// are evaluated once per atom that needs them.  FIRE's P = sum_i v_i . F_i
-// is summed by one lane in atom order.  Expressions follow the reference's
+// Layout: one block per pixel column, the atoms' positions, velocities and
+// force accumulators in shared memory.  The reference sums each atom's force
+// over its interaction list in list order; here every interaction is computed
+// once, into force slots, and every atom has its list of (slot, sign) entries in
+// that same order (built on the host), which one thread per component adds, so
+// every per-atom sum is formed in the reference's order.  FIRE's P = sum_i v_i .
+// F_i is summed by one thread in atom order.  Expressions follow the reference's
 // operation order (vectors.hpp:99-125); the transcendental functions (exp,
 // acos, sin, atan) are CUDA's, so results agree with the reference to
 // rounding, not bit for bit.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -30,7 +29,7 @@ struct mafm_flex {
     mafm_scan_desc d{};
     mafm::ScanParams P{};   // pixel grid, cell, minimiser, tip–dummy terms
     int n_sys = 0;          // atoms incl. dummy (0) and tip (1)
-    int n_bonds = 0, n_angles = 0, n_dihedrals = 0, n_pairs = 0, n_xy = 0, n_ts = 0;
+    int n_ts = 0;
     void* dev_block = nullptr;   // every device array, one allocation
     size_t block_bytes = 0;
     struct Dev {
@@ -47,8 +46,16 @@ struct mafm_flex {
         const void* pair_par;       // FlexPair[n_pairs]
         const double* xy;           // [3 n_xy] atom (as double), x0, y0
         const int* list_begin;      // [n_sys + 1]
-        const int* list;            // entries: kind | role << 8, index
+        const int* list;            // per atom, in the reference's order: slot << 1 | negated
+        const int* warp_begin;      // [kFlexWarps + 1] chunks of every warp
+        const int* chunk_kind;      // [chunks]
+        const int* task;            // [32 chunks] interaction indices, -1: none
+        int slot_base[12];          // first force slot of every kind
+        int n_energies;             // the tip's terms: slots 0 .. n_energies - 1
     } dv{};
+    int n_slots = 0;
+    double* scratch = nullptr;      // energies and slots of every block, when shared memory is too small
+    size_t scratch_doubles = 0;
     mafm::RunCounters* ctr = nullptr;
     mafm::RunCounters* host_ctr = nullptr;
     double sub[6] = {0, 0, 0, 0, 0, 0};   // multiplier, ulj, ushift, z0, rc, sig
@@ -62,6 +69,14 @@ enum : int {
     FT_TS_VDW = 0, FT_TS_COUL, FT_TD_VDW, FT_TD_COUL, FT_TD_HARM, FT_BOND, FT_ANGLE,
     FT_DIHEDRAL, FT_PAIR_VDW, FT_PAIR_COUL, FT_SUBSTRATE, FT_XY
 };
+
+// Force vectors an interaction leaves: one for its first atom (the second gets
+// its negative); an angle's for atom 1, atom 2 and their sum; a dihedral's four.
+__host__ __device__ constexpr int flex_slots(int kind) {
+    return kind == FT_ANGLE ? 3 : kind == FT_DIHEDRAL ? 4 : 1;
+}
+
+constexpr int kFlexWarps = 8;
 
 struct FlexTS {          // one tip–surface term: LJ / Morse (+ the image shift), or Coulomb
     int atom;            // system index of the surface atom
@@ -131,10 +146,13 @@ struct FlexKernelArgs {
     double sub[6];
     double sub_k;
     int n_sys;
+    int n_ts;
+    int n_slots;
     int col_begin, col_end;
     mafm_point* out;
     int state_column;
     double* states;
+    double* scratch;      // energies and force slots of every block, null: shared memory
     unsigned long long watchdog_ns;
     RunCounters* ctr;
 };
@@ -145,420 +163,446 @@ __device__ __forceinline__ unsigned long long now_ns() {
     return t;
 }
 
-// Force (and, for the tip, energy) on atom `a` at positions pe: the atom's
-// entries in list order.  tip_only keeps the tip–surface terms (the output
-// evaluation, System::evalTipSurfaceForces, system.cpp:41-51).
-__device__ V3 atom_force(const FlexKernelArgs& A, const double* pe, int a, bool tip_only, double& e_sum) {
+__device__ __forceinline__ void put3(double* res, int slot, V3 v) {
+    res[3 * slot] = v.x;
+    res[3 * slot + 1] = v.y;
+    res[3 * slot + 2] = v.z;
+}
+
+// One interaction of kind `kind` (all lanes of a warp the same kind): its force
+// vectors into its slots, its energy into e (used for the tip's terms only).
+__device__ void eval_task(const FlexKernelArgs& A, const double* pe, int kind, int idx, double* res,
+                          double* en) {
     const auto& dv = A.dv;
     const FlexTS* ts = static_cast<const FlexTS*>(dv.ts);
     const FlexPair* pp = static_cast<const FlexPair*>(dv.pair_par);
-    V3 F{0, 0, 0};
-    double E = 0;
+    const int slot = dv.slot_base[kind] + idx * flex_slots(kind);
     auto P3 = [&](int i) { return v3(pe + 3 * i); };
-    for (int q = dv.list_begin[a]; q < dv.list_begin[a + 1]; ++q) {
-        const int kr = dv.list[2 * q], idx = dv.list[2 * q + 1];
-        const int kind = kr & 0xff, role = kr >> 8;
-        if (tip_only && kind != FT_TS_VDW && kind != FT_TS_COUL) continue;
-        double e = 0;
-        switch (kind) {
-            case FT_TS_VDW: {   // LJInteraction(1, j, shift) / Morse
-                const FlexTS& t = ts[idx];
-                const V3 sh{t.shift[0], t.shift[1], t.shift[2]};
-                const V3 f = vdw_force(t.kind, t.p, sub3(P3(1), add3(P3(t.atom), sh)), e);
-                F = role == 0 ? add3(F, f) : sub3(F, f);
-                break;
-            }
-            case FT_TS_COUL: {
-                const FlexTS& t = ts[idx];
-                const V3 f = coul_force(t.qq, sub3(P3(1), P3(t.atom)), e);
-                F = role == 0 ? add3(F, f) : sub3(F, f);
-                break;
-            }
-            case FT_TD_VDW: {   // addVDWInteraction(0, 1)
-                const V3 f = vdw_force(A.P.td_kind, A.P.td_p, sub3(P3(0), P3(1)), e);
-                F = role == 0 ? add3(F, f) : sub3(F, f);
-                break;
-            }
-            case FT_TD_COUL: {
-                const V3 f = coul_force(A.P.td_qq, sub3(P3(0), P3(1)), e);
-                F = role == 0 ? add3(F, f) : sub3(F, f);
-                break;
-            }
-            case FT_TD_HARM: {  // TipHarmonicInteraction (interactions.cpp:252-266)
-                const V3 r_vec = sub3(P3(0), P3(1));
-                const double r = sqrt(r_vec.x * r_vec.x + r_vec.y * r_vec.y);
-                const double dr = r - A.P.harm_r0;
-                e = A.P.harm_k * dr * dr;
-                V3 f{0, 0, 0};
-                if (r > 1e-10) {
-                    const double c = -2 * A.P.harm_k * dr / r;
-                    f = V3{c * r_vec.x, c * r_vec.y, 0};
-                }
-                F = role == 0 ? add3(F, f) : sub3(F, f);
-                break;
-            }
-            case FT_BOND: {     // HarmonicInteraction (interactions.cpp:298-309)
-                const int i = dv.bonds[2 * idx], j = dv.bonds[2 * idx + 1];
-                const double k = dv.bond_par[2 * idx], r0 = dv.bond_par[2 * idx + 1];
-                const V3 r_vec = sub3(P3(i), P3(j));
-                const double r = len3(r_vec);
-                const double dr = r - r0;
-                e = k * (dr * dr);
-                const V3 f = scal(-2 * k * dr / r, r_vec);
-                F = role == 0 ? add3(F, f) : sub3(F, f);
-                break;
-            }
-            case FT_ANGLE: {    // HarmonicAngleInteraction (interactions.cpp:311-338)
-                const int sh = dv.angles[3 * idx], i1 = dv.angles[3 * idx + 1], i2 = dv.angles[3 * idx + 2];
-                const double k = dv.angle_par[2 * idx], theta0 = dv.angle_par[2 * idx + 1];
-                const V3 r1_vec = sub3(P3(i1), P3(sh));
-                const V3 r2_vec = sub3(P3(i2), P3(sh));
-                const double r1 = len3(r1_vec), r2 = len3(r2_vec);
-                double cos_t = dot3(r1_vec, r2_vec) / (r1 * r2);
-                if (cos_t > 1) cos_t = 1;
-                else if (cos_t < -1) cos_t = -1;
-                const double theta = acos(cos_t);
-                const double sin_t = sin(theta);
-                const double d_theta = theta - theta0;
-                const double f_mul = -2 * k * d_theta / sin_t;
-                const V3 f1 = scal(-f_mul / r1, sub3(div3(r2_vec, r2), div3(mul3(r1_vec, cos_t), r1)));
-                const V3 f2 = scal(-f_mul / r2, sub3(div3(r1_vec, r1), div3(mul3(r2_vec, cos_t), r2)));
-                e = k * (d_theta * d_theta);
-                if (role == 1) F = add3(F, f1);
-                else if (role == 2) F = add3(F, f2);
-                else F = sub3(F, add3(f1, f2));
-                break;
-            }
-            case FT_DIHEDRAL: { // HarmonicDihedralInteraction (interactions.cpp:340-370)
-                const int* at = dv.dihedrals + 4 * idx;
-                const double k = dv.dihedral_par[2 * idx], sigma0 = dv.dihedral_par[2 * idx + 1];
-                const V3 r12 = sub3(P3(at[0]), P3(at[1]));
-                const V3 r23v = sub3(P3(at[1]), P3(at[2]));
-                const V3 r43 = sub3(P3(at[3]), P3(at[2]));
-                const double r23 = len3(r23v);
-                const V3 m_vec = cross3(r12, r23v);
-                const V3 n_vec = cross3(r43, r23v);
-                const double m = len3(m_vec), n = len3(n_vec);
-                const double tan_s = dot3(n_vec, r12) * r23 / dot3(m_vec, n_vec);
-                const double sigma = atan(tan_s);
-                const double d_sigma = sigma - sigma0;
-                const double f_mul = 2 * k * d_sigma;
-                V3 f;
-                if (role == 0) {
-                    f = scal(-f_mul * r23 / (m * m), m_vec);
-                } else if (role == 1) {
-                    f = scal(-f_mul, sub3(scal(dot3(r43, r23v) / (n * n * r23), n_vec),
-                                          scal(((r23 * r23) + dot3(r12, r23v)) / (m * m * r23), m_vec)));
-                } else if (role == 2) {
-                    f = scal(-f_mul, add3(scal(dot3(r12, r23v) / (m * m * r23), m_vec),
-                                          scal(((r23 * r23) - dot3(r43, r23v)) / (n * n * r23), n_vec)));
-                } else {
-                    f = scal(f_mul * r23 / (n * n), n_vec);
-                }
-                e = k * (d_sigma * d_sigma);
-                F = add3(F, f);
-                break;
-            }
-            case FT_PAIR_VDW: {
-                const int i = dv.pairs[2 * idx], j = dv.pairs[2 * idx + 1];
-                const V3 f = vdw_force(pp[idx].kind, pp[idx].p, sub3(P3(i), P3(j)), e);
-                F = role == 0 ? add3(F, f) : sub3(F, f);
-                break;
-            }
-            case FT_PAIR_COUL: {
-                const int i = dv.pairs[2 * idx], j = dv.pairs[2 * idx + 1];
-                const V3 f = coul_force(pp[idx].qq, sub3(P3(i), P3(j)), e);
-                F = role == 0 ? add3(F, f) : sub3(F, f);
-                break;
-            }
-            case FT_SUBSTRATE: { // SubstrateInteraction (interactions.cpp:280-296)
-                const double dz = pe[3 * a + 2] - A.sub[3];
-                const double sig_z = A.sub[5] / dz;
-                const double sig_z2 = sig_z * sig_z;
-                const double sig_z4 = sig_z2 * sig_z2;
-                const double sig_z10 = sig_z4 * sig_z4 * sig_z2;
-                double fterm = 0.0;
-                if (dz <= A.sub[4]) {
-                    e = A.sub[0] * (2. / 5 * sig_z10 - sig_z4) + A.sub[1] * dz * dz - A.sub[2];
-                    fterm += 4 * A.sub[0] / dz * (sig_z10 - sig_z4) + 2 * A.sub[1] * dz;
-                }
-                F.z += fterm;
-                break;
-            }
-            case FT_XY: {       // XYHarmonicInteraction (interactions.cpp:268-278)
-                const double rx = pe[3 * a] - dv.xy[3 * idx + 1];
-                const double ry = pe[3 * a + 1] - dv.xy[3 * idx + 2];
-                const double r = sqrt(rx * rx + ry * ry);
-                e = A.sub_k * r * r;
-                if (r > 1e-10) {
-                    const double c = -2 * A.sub_k;
-                    F.x += c * rx;
-                    F.y += c * ry;
-                    F.z += 0.0;
-                } else {
-                    F.x += 0.0;
-                    F.y += 0.0;
-                    F.z += 0.0;
-                }
-                break;
-            }
-            default:
-                break;
+    double e = 0;
+    switch (kind) {
+        case FT_TS_VDW: {   // LJInteraction(1, j, shift) / Morse
+            const FlexTS& t = ts[idx];
+            const V3 sh{t.shift[0], t.shift[1], t.shift[2]};
+            put3(res, slot, vdw_force(t.kind, t.p, sub3(P3(1), add3(P3(t.atom), sh)), e));
+            en[slot] = e;
+            break;
         }
-        E += e;
+        case FT_TS_COUL: {
+            const FlexTS& t = ts[idx];
+            put3(res, slot, coul_force(t.qq, sub3(P3(1), P3(t.atom)), e));
+            en[slot] = e;
+            break;
+        }
+        case FT_TD_VDW: {   // addVDWInteraction(0, 1)
+            put3(res, slot, vdw_force(A.P.td_kind, A.P.td_p, sub3(P3(0), P3(1)), e));
+            en[slot] = e;
+            break;
+        }
+        case FT_TD_COUL: {
+            put3(res, slot, coul_force(A.P.td_qq, sub3(P3(0), P3(1)), e));
+            en[slot] = e;
+            break;
+        }
+        case FT_TD_HARM: {  // TipHarmonicInteraction (interactions.cpp:252-266)
+            const V3 r_vec = sub3(P3(0), P3(1));
+            const double r = sqrt(r_vec.x * r_vec.x + r_vec.y * r_vec.y);
+            const double dr = r - A.P.harm_r0;
+            en[slot] = A.P.harm_k * dr * dr;
+            V3 f{0, 0, 0};
+            if (r > 1e-10) {
+                const double c = -2 * A.P.harm_k * dr / r;
+                f = V3{c * r_vec.x, c * r_vec.y, 0};
+            }
+            put3(res, slot, f);
+            break;
+        }
+        case FT_BOND: {     // HarmonicInteraction (interactions.cpp:298-309)
+            const int i = dv.bonds[2 * idx], j = dv.bonds[2 * idx + 1];
+            const double k = dv.bond_par[2 * idx], r0 = dv.bond_par[2 * idx + 1];
+            const V3 r_vec = sub3(P3(i), P3(j));
+            const double r = len3(r_vec);
+            const double dr = r - r0;
+            put3(res, slot, scal(-2 * k * dr / r, r_vec));
+            break;
+        }
+        case FT_ANGLE: {    // HarmonicAngleInteraction (interactions.cpp:311-338)
+            const int sh = dv.angles[3 * idx], i1 = dv.angles[3 * idx + 1], i2 = dv.angles[3 * idx + 2];
+            const double k = dv.angle_par[2 * idx], theta0 = dv.angle_par[2 * idx + 1];
+            const V3 r1_vec = sub3(P3(i1), P3(sh));
+            const V3 r2_vec = sub3(P3(i2), P3(sh));
+            const double r1 = len3(r1_vec), r2 = len3(r2_vec);
+            double cos_t = dot3(r1_vec, r2_vec) / (r1 * r2);
+            if (cos_t > 1) cos_t = 1;
+            else if (cos_t < -1) cos_t = -1;
+            const double theta = acos(cos_t);
+            const double sin_t = sin(theta);
+            const double d_theta = theta - theta0;
+            const double f_mul = -2 * k * d_theta / sin_t;
+            const V3 f1 = scal(-f_mul / r1, sub3(div3(r2_vec, r2), div3(mul3(r1_vec, cos_t), r1)));
+            const V3 f2 = scal(-f_mul / r2, sub3(div3(r1_vec, r1), div3(mul3(r2_vec, cos_t), r2)));
+            put3(res, slot, f1);
+            put3(res, slot + 1, f2);
+            put3(res, slot + 2, add3(f1, f2));
+            break;
+        }
+        case FT_DIHEDRAL: { // HarmonicDihedralInteraction (interactions.cpp:340-370)
+            const int* at = dv.dihedrals + 4 * idx;
+            const double k = dv.dihedral_par[2 * idx], sigma0 = dv.dihedral_par[2 * idx + 1];
+            const V3 r12 = sub3(P3(at[0]), P3(at[1]));
+            const V3 r23v = sub3(P3(at[1]), P3(at[2]));
+            const V3 r43 = sub3(P3(at[3]), P3(at[2]));
+            const double r23 = len3(r23v);
+            const V3 m_vec = cross3(r12, r23v);
+            const V3 n_vec = cross3(r43, r23v);
+            const double m = len3(m_vec), n = len3(n_vec);
+            const double tan_s = dot3(n_vec, r12) * r23 / dot3(m_vec, n_vec);
+            const double sigma = atan(tan_s);
+            const double d_sigma = sigma - sigma0;
+            const double f_mul = 2 * k * d_sigma;
+            put3(res, slot, scal(-f_mul * r23 / (m * m), m_vec));
+            put3(res, slot + 1, scal(-f_mul, sub3(scal(dot3(r43, r23v) / (n * n * r23), n_vec),
+                                                  scal(((r23 * r23) + dot3(r12, r23v)) / (m * m * r23), m_vec))));
+            put3(res, slot + 2, scal(-f_mul, add3(scal(dot3(r12, r23v) / (m * m * r23), m_vec),
+                                                  scal(((r23 * r23) - dot3(r43, r23v)) / (n * n * r23), n_vec))));
+            put3(res, slot + 3, scal(f_mul * r23 / (n * n), n_vec));
+            break;
+        }
+        case FT_PAIR_VDW: {
+            const int i = dv.pairs[2 * idx], j = dv.pairs[2 * idx + 1];
+            put3(res, slot, vdw_force(pp[idx].kind, pp[idx].p, sub3(P3(i), P3(j)), e));
+            break;
+        }
+        case FT_PAIR_COUL: {
+            const int i = dv.pairs[2 * idx], j = dv.pairs[2 * idx + 1];
+            put3(res, slot, coul_force(pp[idx].qq, sub3(P3(i), P3(j)), e));
+            break;
+        }
+        case FT_SUBSTRATE: { // SubstrateInteraction (interactions.cpp:280-296); idx: the atom
+            const double dz = pe[3 * idx + 2] - A.sub[3];
+            const double sig_z = A.sub[5] / dz;
+            const double sig_z2 = sig_z * sig_z;
+            const double sig_z4 = sig_z2 * sig_z2;
+            const double sig_z10 = sig_z4 * sig_z4 * sig_z2;
+            double fterm = 0.0;
+            if (dz <= A.sub[4]) fterm += 4 * A.sub[0] / dz * (sig_z10 - sig_z4) + 2 * A.sub[1] * dz;
+            // -0: adding it leaves x and y as they are, signed zeros too
+            put3(res, slot, V3{-0.0, -0.0, fterm});
+            break;
+        }
+        case FT_XY: {       // XYHarmonicInteraction (interactions.cpp:268-278)
+            const int a = (int)dv.xy[3 * idx];
+            const double rx = pe[3 * a] - dv.xy[3 * idx + 1];
+            const double ry = pe[3 * a + 1] - dv.xy[3 * idx + 2];
+            const double r = sqrt(rx * rx + ry * ry);
+            const double c = -2 * A.sub_k;
+            put3(res, slot, r > 1e-10 ? V3{c * rx, c * ry, 0.0} : V3{0.0, 0.0, 0.0});
+            break;
+        }
+        default:
+            break;
     }
-    e_sum = E;
-    return F;
 }
 
-// Per-warp shared arrays, 3 doubles per atom each.
+// Shared arrays of a block, 3 doubles per atom each.
 struct Slice {
     double* pos;   // positions_
     double* vel;   // velocities_
-    double* pe;    // positions of the current evaluation
+    double* pe;    // positions of the current evaluation; the mixed velocities
     double* vk;    // RK4 v_k / midpoint v2
     double* fsum;  // RK4 force sum; forces_ of the last step otherwise
     double* vsum;  // RK4 velocity sum
     double* f;     // forces of the current evaluation
+    double* dot;   // v_i . F_i
+    double* en;    // energies of the tip's terms
+    double* res;   // force slots
 };
 
-__global__ void flex_kernel(FlexKernelArgs A) {
+// What one thread decides for the block.
+struct FlexCtl {
+    double dt, alpha, e_tip, pw, e_eval;
+    double ft[3];
+    int conv, n_non_neg, col;
+};
+
+// One block of kFlexWarps warps relaxes one column.  An FP64 instruction of a
+// warp takes 64 cycles whatever its lanes do, and an SM starts one every 19, so
+// what counts is the number of warp instructions on the longest chain.  An
+// evaluation therefore computes every interaction once, 32 of one kind to a
+// warp, the kinds' chunks dealt to the warps by cost, into slots of shared
+// memory; then one thread per atom and component adds the atom's slots in the
+// reference's order.  The minimiser's per-atom parts run one thread per
+// component, beside the convergence test on one warp and the power P on
+// another.  A flexible C10H8 + H2 (25 columns x 6 heights): 505 -> 19.3 ms;
+// before, a warp held a column, each lane evaluated its atoms' interactions
+// one after another (the tip's 43 on one lane), and the kinds diverged.
+__global__ void __launch_bounds__(32 * kFlexWarps) flex_kernel(const __grid_constant__ FlexKernelArgs A) {
     extern __shared__ __align__(16) double flex_smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int na = A.n_sys;
-    const size_t per = (size_t)na * 3;
-    double* base = flex_smem + (size_t)warp * 7 * per;
+    __shared__ FlexCtl ctl;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int kThreads = 32 * kFlexWarps;
+    const int na = A.n_sys, nq = 3 * na;
+    const size_t per = (size_t)nq;
+    double* base = flex_smem;
     Slice S{base, base + per, base + 2 * per, base + 3 * per, base + 4 * per, base + 5 * per,
-            base + 6 * per};
-    __shared__ int s_col[32];
+            base + 6 * per, base + 7 * per, base + 7 * per + na, nullptr};
+    if (A.scratch) S.en = A.scratch + (size_t)blockIdx.x * (A.dv.n_energies + 3 * (size_t)A.n_slots);
+    S.res = S.en + A.dv.n_energies;
     const ScanParams& P = A.P;
+    const auto& dv = A.dv;
     const unsigned long long t0 = now_ns();
-    unsigned long long my_steps = 0, my_evals = 0;
+    unsigned long long my_steps = 0, my_evals = 0;   // thread 0
     unsigned err = 0;
-    const int* fixed = A.dv.fixed;
+    const int* fixed = dv.fixed;
+    auto late = [&]() { return __syncthreads_or(tid == 0 && now_ns() - t0 > A.watchdog_ns) != 0; };
+
+    // Forces at positions src into S.f and the tip's energy into ctl.e_eval;
+    // tip_only: the tip–surface terms alone (System::evalTipSurfaceForces,
+    // system.cpp:41-51), summed for the tip into ctl.ft.  Starts and ends with
+    // a block barrier.
+    auto evaluate = [&](const double* src, bool tip_only) {
+        __syncthreads();
+        for (int c = dv.warp_begin[warp]; c < dv.warp_begin[warp + 1]; ++c) {
+            const int kind = dv.chunk_kind[c];
+            if (tip_only && kind != FT_TS_VDW && kind != FT_TS_COUL) continue;
+            const int idx = dv.task[32 * c + lane];
+            if (idx >= 0) eval_task(A, src, kind, idx, S.res, S.en);
+        }
+        __syncthreads();
+        const int n_f = tip_only ? 3 : nq;
+        for (int q = tid; q < n_f; q += kThreads) {
+            const int a = tip_only ? 1 : q / 3, d = tip_only ? q : q - 3 * a;
+            double acc = 0;
+            for (int i = dv.list_begin[a]; i < dv.list_begin[a + 1]; ++i) {
+                const int s = dv.list[i];
+                if (tip_only && (s >> 1) >= A.n_ts) continue;
+                const double v = S.res[3 * (s >> 1) + d];
+                acc += (s & 1) ? -v : v;
+            }
+            if (tip_only) ctl.ft[d] = acc;
+            else S.f[q] = acc;
+        }
+        if (tid == kThreads - 1) {
+            double E = 0;
+            for (int i = dv.list_begin[1]; i < dv.list_begin[2]; ++i) {
+                const int s = dv.list[i] >> 1;
+                if (!(tip_only && s >= A.n_ts)) E += S.en[s];
+            }
+            ctl.e_eval = E;
+        }
+        if (tid == 0 && !tip_only) my_evals += 1;
+        __syncthreads();
+    };
 
     for (;;) {
-        if (lane == 0) {
+        __syncthreads();
+        if (tid == 0) {
             const unsigned long long t = atomicAdd(&A.ctr->next_work, 1ull);
-            s_col[warp] = (t < (unsigned long long)(A.col_end - A.col_begin)) ? A.col_begin + (int)t : -1;
+            ctl.col = (t < (unsigned long long)(A.col_end - A.col_begin)) ? A.col_begin + (int)t : -1;
         }
-        __syncwarp();
-        const int col = s_col[warp];
-        __syncwarp();
+        __syncthreads();
+        const int col = ctl.col;
         if (col < 0) break;
-        if (__any_sync(0xffffffffu, now_ns() - t0 > A.watchdog_ns)) {
+        if (late()) {
             err |= ERR_WATCHDOG;
             break;
         }
         // System min_system = system (simulation.cpp:93): the initial state
-        for (int a = lane; a < na; a += 32)
-            for (int d = 0; d < 3; ++d) {
-                S.pos[3 * a + d] = A.dv.pos0[3 * a + d];
-                S.vel[3 * a + d] = 0.0;
-                S.fsum[3 * a + d] = 0.0;
-            }
-        __syncwarp();
-        // setDummyXY / setDummyZ (system.cpp:139-162, system.hpp:46-49)
-        const int i = col / P.ny, j = col % P.ny;
-        double x = i * P.dx, y = j * P.dy;
-        if (P.tip_pbc) {
-            const double* ci = P.cell_inv;
-            const double* c = P.cell;
-            const double tx = x - P.offset[0], ty = y - P.offset[1], tz = 0 - P.offset[2];
-            double cx = ci[0] * tx + ci[1] * ty + ci[2] * tz;
-            double cy = ci[3] * tx + ci[4] * ty + ci[5] * tz;
-            const double cz = ci[6] * tx + ci[7] * ty + ci[8] * tz;
-            cx -= floor(cx);
-            cy -= floor(cy);
-            x = (c[0] * cx + c[1] * cy + c[2] * cz) + P.offset[0];
-            y = (c[3] * cx + c[4] * cy + c[5] * cz) + P.offset[1];
+        for (int q = tid; q < nq; q += kThreads) {
+            S.pos[q] = dv.pos0[q];
+            S.vel[q] = 0.0;
+            S.fsum[q] = 0.0;
         }
-        if (lane == 0) {
+        __syncthreads();
+        if (tid == 0) {
+            // setDummyXY / setDummyZ (system.cpp:139-162, system.hpp:46-49)
+            const int i = col / P.ny, j = col % P.ny;
+            double x = i * P.dx, y = j * P.dy;
+            if (P.tip_pbc) {
+                const double* ci = P.cell_inv;
+                const double* c = P.cell;
+                const double tx = x - P.offset[0], ty = y - P.offset[1], tz = 0 - P.offset[2];
+                double cx = ci[0] * tx + ci[1] * ty + ci[2] * tz;
+                double cy = ci[3] * tx + ci[4] * ty + ci[5] * tz;
+                const double cz = ci[6] * tx + ci[7] * ty + ci[8] * tz;
+                cx -= floor(cx);
+                cy -= floor(cy);
+                x = (c[0] * cx + c[1] * cy + c[2] * cz) + P.offset[0];
+                y = (c[3] * cx + c[4] * cy + c[5] * cz) + P.offset[1];
+            }
             S.pos[0] = x; S.pos[1] = y; S.pos[2] = P.zhigh;
             S.pos[3] = x; S.pos[4] = y; S.pos[5] = P.zhigh - P.tip_dummy_d;
+            ctl.e_tip = 0.0;   // System::energies_[1], carried between heights
         }
-        __syncwarp();
-        double e_tip = 0.0;   // System::energies_[1], carried between heights
         for (int k = 0; k < P.nz; ++k) {
             // ---- FIREMinimisation / SDMinimisation (minimiser.cpp:39-129) ----
-            double alpha = 0.1, dt = P.dt;
-            const double dt_max = 10 * P.dt;
-            int n_non_neg = 0;
+            __syncthreads();
+            if (tid == 0) {
+                ctl.alpha = 0.1;
+                ctl.dt = P.dt;
+                ctl.n_non_neg = 0;
+            }
             int n = 1;
             for (; n < P.maxsteps; ++n) {
-                if (((n & 1023) == 0) && __any_sync(0xffffffffu, now_ns() - t0 > A.watchdog_ns)) {
+                if ((n & 1023) == 0 && late()) {
                     err |= ERR_WATCHDOG;
                     break;
                 }
-                const double prev_tip_e = e_tip;
-                double e_new = 0.0;
-                // evaluation at positions src into S.f; returns the tip energy
-                auto evaluate = [&](const double* src) {
-                    double et = 0.0;
-                    for (int a = lane; a < na; a += 32) {
-                        double e;
-                        const V3 F = atom_force(A, src, a, false, e);
-                        S.f[3 * a] = F.x; S.f[3 * a + 1] = F.y; S.f[3 * a + 2] = F.z;
-                        if (a == 1) et = e;
-                    }
-                    __syncwarp();
-                    my_evals += (lane == 0);
-                    return __shfl_sync(0xffffffffu, et, 1);
-                };
+                double e1 = 0, e2 = 0, e3 = 0;
+                evaluate(S.pos, false);
+                const double dt = ctl.dt;
                 if (P.minimiser == MAFM_MIN_SD) {
-                    e_new = evaluate(S.pos);
-                    for (int a = lane; a < na; a += 32)
-                        for (int d = 0; d < 3; ++d) S.fsum[3 * a + d] = S.f[3 * a + d];
+                    for (int q = tid; q < nq; q += kThreads) S.fsum[q] = S.f[q];
                 } else if (P.integrator == MAFM_INT_EULER) {
-                    e_new = evaluate(S.pos);
-                    for (int a = lane; a < na; a += 32) {
-                        for (int d = 0; d < 3; ++d) S.fsum[3 * a + d] = S.f[3 * a + d];
-                        if (fixed[a] != 1)
-                            for (int d = 0; d < 3; ++d) {
-                                S.pos[3 * a + d] += dt * S.vel[3 * a + d];
-                                S.vel[3 * a + d] += dt * S.f[3 * a + d] / 1.0;
-                            }
+                    for (int q = tid; q < nq; q += kThreads) {
+                        S.fsum[q] = S.f[q];
+                        if (fixed[q / 3] != 1) {
+                            S.pos[q] += dt * S.vel[q];
+                            S.vel[q] += dt * S.f[q];
+                        }
                     }
                 } else if (P.integrator == MAFM_INT_MIDPOINT) {
-                    (void)evaluate(S.pos);
-                    for (int a = lane; a < na; a += 32)
-                        for (int d = 0; d < 3; ++d) {
-                            S.pe[3 * a + d] = S.pos[3 * a + d];
-                            S.vk[3 * a + d] = S.vel[3 * a + d];
-                            if (fixed[a] != 1) {
-                                S.pe[3 * a + d] += dt / 2 * S.vel[3 * a + d];
-                                S.vk[3 * a + d] += dt / 2 * S.f[3 * a + d] / 1.0;
-                            }
+                    for (int q = tid; q < nq; q += kThreads) {
+                        double p2 = S.pos[q], v2 = S.vel[q];
+                        if (fixed[q / 3] != 1) {
+                            p2 += dt / 2 * S.vel[q];
+                            v2 += dt / 2 * S.f[q];
                         }
-                    __syncwarp();
-                    e_new = evaluate(S.pe);
-                    for (int a = lane; a < na; a += 32)
-                        for (int d = 0; d < 3; ++d) {
-                            if (fixed[a] != 1) {
-                                S.pos[3 * a + d] += dt * S.vk[3 * a + d];
-                                S.vel[3 * a + d] += dt * S.f[3 * a + d] / 1.0;
-                            }
-                            S.fsum[3 * a + d] = S.f[3 * a + d];
+                        S.pe[q] = p2;
+                        S.vk[q] = v2;
+                    }
+                    evaluate(S.pe, false);
+                    for (int q = tid; q < nq; q += kThreads) {
+                        if (fixed[q / 3] != 1) {
+                            S.pos[q] += dt * S.vk[q];
+                            S.vel[q] += dt * S.f[q];
                         }
+                        S.fsum[q] = S.f[q];
+                    }
                 } else {   // RK4 (integrators.cpp:56-111)
-                    const double e1 = evaluate(S.pos);
-                    for (int a = lane; a < na; a += 32)
-                        for (int d = 0; d < 3; ++d) {
-                            const int q = 3 * a + d;
-                            S.fsum[q] = S.f[q];                 // f1
-                            S.vsum[q] = S.vel[q];               // v
-                            S.pe[q] = S.pos[q];
-                            S.vk[q] = S.vel[q];
-                            if (fixed[a] != 1) {
-                                S.pe[q] += dt / 2 * S.vel[q];   // p2
-                                S.vk[q] += dt / 2 * S.f[q] / 1.0;   // v2
-                            }
+                    e1 = ctl.e_eval;
+                    for (int q = tid; q < nq; q += kThreads) {
+                        S.fsum[q] = S.f[q];                 // f1
+                        S.vsum[q] = S.vel[q];               // v
+                        double p2 = S.pos[q], v2 = S.vel[q];
+                        if (fixed[q / 3] != 1) {
+                            p2 += dt / 2 * S.vel[q];
+                            v2 += dt / 2 * S.f[q];
                         }
-                    __syncwarp();
-                    const double e2 = evaluate(S.pe);
-                    for (int a = lane; a < na; a += 32)
-                        for (int d = 0; d < 3; ++d) {
-                            const int q = 3 * a + d;
-                            S.fsum[q] = S.fsum[q] + 2 * S.f[q];
-                            S.vsum[q] = S.vsum[q] + 2 * S.vk[q];
-                            const double v2 = S.vk[q];
-                            S.pe[q] = S.pos[q];
-                            S.vk[q] = S.vel[q];
-                            if (fixed[a] != 1) {
-                                S.pe[q] += dt / 2 * v2;             // p3
-                                S.vk[q] += dt / 2 * S.f[q] / 1.0;   // v3
-                            }
+                        S.pe[q] = p2;
+                        S.vk[q] = v2;
+                    }
+                    evaluate(S.pe, false);
+                    e2 = ctl.e_eval;
+                    for (int q = tid; q < nq; q += kThreads) {
+                        S.fsum[q] = S.fsum[q] + 2 * S.f[q];
+                        S.vsum[q] = S.vsum[q] + 2 * S.vk[q];
+                        const double v2 = S.vk[q];
+                        double p3 = S.pos[q], v3 = S.vel[q];
+                        if (fixed[q / 3] != 1) {
+                            p3 += dt / 2 * v2;
+                            v3 += dt / 2 * S.f[q];
                         }
-                    __syncwarp();
-                    const double e3 = evaluate(S.pe);
-                    for (int a = lane; a < na; a += 32)
-                        for (int d = 0; d < 3; ++d) {
-                            const int q = 3 * a + d;
-                            S.fsum[q] = S.fsum[q] + 2 * S.f[q];
-                            S.vsum[q] = S.vsum[q] + 2 * S.vk[q];
-                            const double v3 = S.vk[q];
-                            S.pe[q] = S.pos[q];
-                            S.vk[q] = S.vel[q];
-                            if (fixed[a] != 1) {
-                                S.pe[q] += dt * v3;             // p4
-                                S.vk[q] += dt * S.f[q] / 1.0;   // v4
-                            }
+                        S.pe[q] = p3;
+                        S.vk[q] = v3;
+                    }
+                    evaluate(S.pe, false);
+                    e3 = ctl.e_eval;
+                    for (int q = tid; q < nq; q += kThreads) {
+                        S.fsum[q] = S.fsum[q] + 2 * S.f[q];
+                        S.vsum[q] = S.vsum[q] + 2 * S.vk[q];
+                        const double v3 = S.vk[q];
+                        double p4 = S.pos[q], v4 = S.vel[q];
+                        if (fixed[q / 3] != 1) {
+                            p4 += dt * v3;
+                            v4 += dt * S.f[q];
                         }
-                    __syncwarp();
-                    const double e4 = evaluate(S.pe);
-                    for (int a = lane; a < na; a += 32)
-                        for (int d = 0; d < 3; ++d) {
-                            const int q = 3 * a + d;
-                            const double fs = S.fsum[q] + S.f[q];    // f1 + 2f2 + 2f3 + f4
-                            const double vs = S.vsum[q] + S.vk[q];   // v + 2v2 + 2v3 + v4
-                            if (fixed[a] != 1) {
-                                S.pos[q] += dt / 6 * vs;
-                                S.vel[q] += dt / 6 * fs / 1.0;
-                            }
-                            S.fsum[q] = fs / 6;
+                        S.pe[q] = p4;
+                        S.vk[q] = v4;
+                    }
+                    evaluate(S.pe, false);
+                    for (int q = tid; q < nq; q += kThreads) {
+                        const double fs = S.fsum[q] + S.f[q];    // f1 + 2f2 + 2f3 + f4
+                        const double vs = S.vsum[q] + S.vk[q];   // v + 2v2 + 2v3 + v4
+                        if (fixed[q / 3] != 1) {
+                            S.pos[q] += dt / 6 * vs;
+                            S.vel[q] += dt / 6 * fs;
                         }
-                    e_new = (e1 + 2 * e2 + 2 * e3 + e4) / 6;
+                        S.fsum[q] = fs / 6;
+                    }
                 }
-                __syncwarp();
-                e_tip = e_new;
-                // checkConvergence on the tip (minimiser.cpp:15-37)
-                const V3 ft = v3(S.fsum + 3);
-                const double fl = len3(ft);
-                const double ediff = e_tip - prev_tip_e;
-                bool conv;
-                if (P.minterm == MAFM_TERM_E) conv = fabs(ediff) < P.etol;
-                else if (P.minterm == MAFM_TERM_F) conv = fl < P.ftol;
-                else conv = fabs(ediff) < P.etol && fl < P.ftol;
-                if (conv) break;
+                __syncthreads();
+                // beside one another: the convergence test (the last warp), the
+                // power P (the last warp but one), the mixing (the others)
+                if (warp == kFlexWarps - 1) {
+                    if (lane == 0) {
+                        // checkConvergence on the tip (minimiser.cpp:15-37)
+                        const bool rk4 = P.minimiser != MAFM_MIN_SD && P.integrator == MAFM_INT_RK4;
+                        const double e_new = rk4 ? (e1 + 2 * e2 + 2 * e3 + ctl.e_eval) / 6 : ctl.e_eval;
+                        const double ediff = e_new - ctl.e_tip;
+                        bool conv;
+                        if (P.minterm == MAFM_TERM_E) conv = fabs(ediff) < P.etol;
+                        else {
+                            conv = len3(v3(S.fsum + 3)) < P.ftol;
+                            if (P.minterm != MAFM_TERM_F) conv = conv && fabs(ediff) < P.etol;
+                        }
+                        ctl.e_tip = e_new;
+                        ctl.conv = conv;
+                    }
+                } else if (P.minimiser != MAFM_MIN_SD) {
+                    if (warp == kFlexWarps - 2) {
+                        // P = sum_i v_i . F_i in atom order
+                        for (int a = lane; a < na; a += 32)
+                            S.dot[a] = dot3(v3(S.vel + 3 * a), v3(S.fsum + 3 * a));
+                        __syncwarp();
+                        if (lane == 0) {
+                            double pw = 0;
+                            for (int a = 0; a < na; ++a) pw += S.dot[a];
+                            ctl.pw = pw;
+                        }
+                    } else {
+                        // (1 - alpha) v + alpha F.normalized() |v|  (minimiser.cpp:112-113)
+                        const double alpha = ctl.alpha;
+                        for (int q = tid; q < nq; q += kThreads - 64) {
+                            const int a = q / 3;
+                            if (fixed[a] == 1) {
+                                S.pe[q] = S.vel[q];
+                                continue;
+                            }
+                            const double lf = len3(v3(S.fsum + 3 * a));
+                            const double fh = lf > 1e-10 ? S.fsum[q] / lf : 0.0;
+                            S.pe[q] = (1 - alpha) * S.vel[q] + (alpha * fh) * len3(v3(S.vel + 3 * a));
+                        }
+                    }
+                }
+                __syncthreads();
+                if (ctl.conv) break;
                 if (P.minimiser == MAFM_MIN_SD) {
-                    for (int a = lane; a < na; a += 32)
-                        if (fixed[a] != 1)
-                            for (int d = 0; d < 3; ++d) S.pos[3 * a + d] += P.dt * S.fsum[3 * a + d];
-                    __syncwarp();
+                    for (int q = tid; q < nq; q += kThreads)
+                        if (fixed[q / 3] != 1) S.pos[q] += P.dt * S.fsum[q];
                     continue;
                 }
-                // FIRE: P = sum_i v_i . F_i in atom order, then the mixing
-                double pw = 0;
-                if (lane == 0)
-                    for (int a = 0; a < na; ++a) pw += dot3(v3(S.vel + 3 * a), v3(S.fsum + 3 * a));
-                pw = __shfl_sync(0xffffffffu, pw, 0);
-                __syncwarp();
-                for (int a = lane; a < na; a += 32) {
-                    if (fixed[a] == 1) continue;
-                    // (1 - alpha) v + alpha F.normalized() |v|  (minimiser.cpp:112-113)
-                    const V3 v = v3(S.vel + 3 * a);
-                    const V3 mixed = add3(scal(1 - alpha, v),
-                                          mul3(scal(alpha, normalized3(v3(S.fsum + 3 * a))), len3(v)));
-                    S.vel[3 * a] = mixed.x;
-                    S.vel[3 * a + 1] = mixed.y;
-                    S.vel[3 * a + 2] = mixed.z;
-                }
-                __syncwarp();
-                if (pw < 0) {
-                    for (int a = lane; a < na; a += 32)
-                        for (int d = 0; d < 3; ++d) S.vel[3 * a + d] = 0.0;
-                    n_non_neg = 0;
-                    dt *= 0.5;
-                    alpha = 0.1;
-                } else {
-                    if (n_non_neg > 5) {
-                        dt = fmin(dt * 1.1, dt_max);
-                        alpha *= 0.99;
+                const bool neg = ctl.pw < 0;
+                for (int q = tid; q < nq; q += kThreads) S.vel[q] = neg ? 0.0 : S.pe[q];
+                if (tid == kThreads - 1) {
+                    if (neg) {
+                        ctl.n_non_neg = 0;
+                        ctl.dt = ctl.dt * 0.5;
+                        ctl.alpha = 0.1;
+                    } else {
+                        if (ctl.n_non_neg > 5) {
+                            ctl.dt = fmin(ctl.dt * 1.1, 10 * P.dt);
+                            ctl.alpha *= 0.99;
+                        }
+                        ctl.n_non_neg++;
                     }
-                    n_non_neg++;
                 }
-                __syncwarp();
             }
             if (err & ERR_WATCHDOG) break;
             // System::getOutput (system.cpp:28-51)
-            double et = 0;
-            V3 ft{0, 0, 0};
-            if (lane == 1) ft = atom_force(A, S.pos, 1, true, et);
-            et = __shfl_sync(0xffffffffu, et, 1);
-            ft.x = __shfl_sync(0xffffffffu, ft.x, 1);
-            ft.y = __shfl_sync(0xffffffffu, ft.y, 1);
-            ft.z = __shfl_sync(0xffffffffu, ft.z, 1);
-            if (lane == 0) {
+            evaluate(S.pos, true);
+            if (tid == 0) {
+                const double et = ctl.e_eval;
+                const V3 ft = v3(ctl.ft);
                 int st = n >= P.maxsteps ? MAFM_PT_MAXSTEPS : 0;
                 if (!isfinite(ft.x) || !isfinite(ft.y) || !isfinite(ft.z) || !isfinite(et))
                     st |= MAFM_PT_NONFINITE;
@@ -572,30 +616,23 @@ __global__ void flex_kernel(FlexKernelArgs A) {
                 my_steps += (unsigned long long)n;
             }
             if (A.states && col == A.state_column)
-                for (int a = lane; a < na; a += 32)
-                    for (int d = 0; d < 3; ++d) A.states[((size_t)k * na + a) * 3 + d] = S.pos[3 * a + d];
-            __syncwarp();
+                for (int q = tid; q < nq; q += kThreads) A.states[(size_t)k * nq + q] = S.pos[q];
+            __syncthreads();
             // System::lowerTip (system.hpp:51-54)
-            if (lane == 0) {
+            if (tid == 0) {
                 S.pos[2] -= P.dz;
                 S.pos[5] -= P.dz;
             }
-            __syncwarp();
             // the time limit once per height too: a height usually converges in
             // far fewer than the 1024 steps between the checks above
-            if (__any_sync(0xffffffffu, now_ns() - t0 > A.watchdog_ns)) {
+            if (late()) {
                 err |= ERR_WATCHDOG;
                 break;
             }
         }
         if (err & ERR_WATCHDOG) break;
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        my_steps += __shfl_xor_sync(0xffffffffu, my_steps, off);
-        my_evals += __shfl_xor_sync(0xffffffffu, my_evals, off);
-        err |= __shfl_xor_sync(0xffffffffu, err, off);
-    }
-    if (lane == 0) {
+    if (tid == 0) {
         atomicAdd(&A.ctr->total_steps, my_steps);
         atomicAdd(&A.ctr->force_evals, my_evals);
         if (err) atomicOr(&A.ctr->error_word, err);
@@ -666,8 +703,13 @@ extern "C" int mafm_flex_create(int device, const mafm_scan_desc* d, const mafm_
             std::vector<int> fixed(na, 0);
             fixed[0] = 1;
             for (int a = 0; a < ns; ++a) fixed[a + 2] = f->fixed[a];
-            std::vector<std::vector<std::pair<int, int>>> lists(na);   // (kind | role << 8, index)
-            auto add = [&](int atom, int kind, int role, int idx) { lists[atom].push_back({kind | (role << 8), idx}); };
+            struct Entry { int kind, role, idx; };
+            std::vector<std::vector<Entry>> lists(na);
+            std::vector<std::vector<int>> tasks(FT_XY + 1);   // interactions of every kind
+            auto add = [&](int atom, int kind, int role, int idx) {
+                lists[atom].push_back({kind, role, idx});
+                if (tasks[kind].empty() || tasks[kind].back() != idx) tasks[kind].push_back(idx);
+            };
             std::vector<FlexTS> ts;
             // buildTipSurfaceInteractions (simulation.cpp:297-320)
             const int images = d->vdw_pbc ? 9 : 1;
@@ -766,22 +808,63 @@ extern "C" int mafm_flex_create(int device, const mafm_scan_desc* d, const mafm_
             s->sub_k = f->substrate[4];
             std::vector<double> xy;
             for (int a = 2; a < na; ++a) {
-                add(a, FT_SUBSTRATE, 0, 0);
+                add(a, FT_SUBSTRATE, 0, a);
                 if (fixed[a] == 2) {
                     xy.insert(xy.end(), {(double)a, pos0[3 * (size_t)a], pos0[3 * (size_t)a + 1]});
                     add(a, FT_XY, 0, (int)xy.size() / 3 - 1);
                 }
             }
-            // the (kind, index) entries of every atom, atom after atom
+            // force slots, kind after kind: the tip's terms first (both kinds of
+            // tip–surface terms index one list)
+            const int n_ts = (int)ts.size();
+            const int count[12] = {0, n_ts, 1, 1, 1, f->n_bonds, f->n_angles, f->n_dihedrals,
+                                   f->n_pairs, f->n_pairs, na, (int)xy.size() / 3};
+            int slots = 0;
+            for (int kd = FT_TS_VDW; kd <= FT_XY; ++kd) {
+                s->dv.slot_base[kd] = slots;
+                slots += count[kd] * flex_slots(kd);
+                if (kd == FT_TD_HARM) s->dv.n_energies = slots;
+            }
+            s->n_slots = slots;
+            // every atom's slots in the reference's order: a pair's second atom
+            // (role 1; of the dummy's terms the tip, of an angle the shared atom,
+            // role 0) takes the negative
             std::vector<int> begin(na + 1, 0), list;
             for (int a = 0; a < na; ++a) {
-                begin[a] = (int)list.size() / 2;
-                for (const auto& e : lists[a]) list.insert(list.end(), {e.first, e.second});
+                begin[a] = (int)list.size();
+                for (const Entry& e : lists[a]) {
+                    const int first = s->dv.slot_base[e.kind] + e.idx * flex_slots(e.kind);
+                    if (e.kind == FT_ANGLE) list.push_back(e.role == 0 ? (first + 2) << 1 | 1 : (first + e.role - 1) << 1);
+                    else if (e.kind == FT_DIHEDRAL) list.push_back((first + e.role) << 1);
+                    else list.push_back(first << 1 | (e.role == 1));
+                }
             }
-            begin[na] = (int)list.size() / 2;
-            s->n_ts = (int)ts.size();
-            s->n_bonds = f->n_bonds; s->n_angles = f->n_angles; s->n_dihedrals = f->n_dihedrals;
-            s->n_pairs = f->n_pairs; s->n_xy = (int)xy.size() / 3;
+            begin[na] = (int)list.size();
+            // chunks of up to 32 interactions of one kind, the costliest first,
+            // each to the warp with the least to do (costs: FP64 instructions)
+            const int cost[12] = {48, 30, 50, 30, 25, 32, 180, 220, 48, 30, 35, 18};
+            std::vector<std::pair<int, int>> chunks;   // kind, first task
+            for (int kd = FT_TS_VDW; kd <= FT_XY; ++kd)
+                for (size_t i = 0; i < tasks[kd].size(); i += 32) chunks.push_back({kd, (int)i});
+            std::stable_sort(chunks.begin(), chunks.end(),
+                             [&](const auto& x, const auto& y) { return cost[x.first] > cost[y.first]; });
+            std::vector<std::vector<std::pair<int, int>>> of_warp(kFlexWarps);
+            std::vector<long long> load(kFlexWarps, 0);
+            for (const auto& c : chunks) {
+                const size_t w = std::min_element(load.begin(), load.end()) - load.begin();
+                of_warp[w].push_back(c);
+                load[w] += cost[c.first];
+            }
+            std::vector<int> warp_begin(1, 0), chunk_kind, task;
+            for (const auto& w : of_warp) {
+                for (const auto& c : w) {
+                    chunk_kind.push_back(c.first);
+                    for (size_t i = c.second; i < (size_t)c.second + 32; ++i)
+                        task.push_back(i < tasks[c.first].size() ? tasks[c.first][i] : -1);
+                }
+                warp_begin.push_back((int)chunk_kind.size());
+            }
+            s->n_ts = n_ts;
 
             // one device block for every array (256-byte aligned pieces)
             struct Piece { const void* src; size_t bytes; size_t off; };
@@ -807,6 +890,9 @@ extern "C" int mafm_flex_create(int device, const mafm_scan_desc* d, const mafm_
             const size_t o_xy = piece(xy.data(), xy.size() * sizeof(double));
             const size_t o_lb = piece(begin.data(), begin.size() * sizeof(int));
             const size_t o_l = piece(list.data(), list.size() * sizeof(int));
+            const size_t o_wb = piece(warp_begin.data(), warp_begin.size() * sizeof(int));
+            const size_t o_ck = piece(chunk_kind.data(), chunk_kind.size() * sizeof(int));
+            const size_t o_tk = piece(task.data(), task.size() * sizeof(int));
             s->block_bytes = std::max<size_t>(off, 256);
             cuda_check(cudaMalloc(&s->dev_block, s->block_bytes), "cudaMalloc");
             char* dev = static_cast<char*>(s->dev_block);
@@ -827,6 +913,9 @@ extern "C" int mafm_flex_create(int device, const mafm_scan_desc* d, const mafm_
             s->dv.xy = reinterpret_cast<const double*>(dev + o_xy);
             s->dv.list_begin = reinterpret_cast<const int*>(dev + o_lb);
             s->dv.list = reinterpret_cast<const int*>(dev + o_l);
+            s->dv.warp_begin = reinterpret_cast<const int*>(dev + o_wb);
+            s->dv.chunk_kind = reinterpret_cast<const int*>(dev + o_ck);
+            s->dv.task = reinterpret_cast<const int*>(dev + o_tk);
             cuda_check(cudaMalloc(&s->ctr, sizeof(RunCounters)), "cudaMalloc");
             cuda_check(cudaMallocHost(&s->host_ctr, sizeof(RunCounters)), "cudaMallocHost");
         } catch (...) {
@@ -844,6 +933,7 @@ extern "C" int mafm_flex_destroy(mafm_flex* s) {
     if (s) {
         cudaSetDevice(s->device);
         if (s->dev_block) cudaFree(s->dev_block);
+        if (s->scratch) cudaFree(s->scratch);
         if (s->ctr) cudaFree(s->ctr);
         if (s->host_ctr) cudaFreeHost(s->host_ctr);
         delete s;
@@ -910,6 +1000,8 @@ extern "C" int mafm_flex_run(mafm_flex* s, int32_t col_begin, int32_t col_end, m
         std::memcpy(A.sub, s->sub, sizeof A.sub);
         A.sub_k = s->sub_k;
         A.n_sys = s->n_sys;
+        A.n_ts = s->n_ts;
+        A.n_slots = s->n_slots;
         A.col_begin = col_begin;
         A.col_end = col_end;
         A.out = dout;
@@ -918,16 +1010,29 @@ extern "C" int mafm_flex_run(mafm_flex* s, int32_t col_begin, int32_t col_end, m
         A.watchdog_ns = watchdog_ns_from_env();
         A.ctr = s->ctr;
         cuda_check(cudaMemsetAsync(s->ctr, 0, sizeof(RunCounters), st), "reset counters");
-        const size_t per_warp = (size_t)7 * s->n_sys * 3 * sizeof(double);
-        int warps = (int)std::min<size_t>(4, std::max<size_t>(1, (200u * 1024u) / per_warp));
-        const size_t smem = per_warp * warps;
+        // the atoms' arrays and v.F; the tip's energies and the force slots
+        // while they fit (about 8,000 slots), else in global memory
+        const size_t atom_bytes = (size_t)22 * s->n_sys * sizeof(double);
+        const size_t block_doubles = (size_t)s->dv.n_energies + 3 * (size_t)s->n_slots;
+        const bool in_smem = atom_bytes + block_doubles * sizeof(double) <= 200u * 1024u;
+        const size_t smem = atom_bytes + (in_smem ? block_doubles * sizeof(double) : 0);
         cuda_check(cudaFuncSetAttribute(flex_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                    "flex smem");
+        int per_sm = 0;
+        cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, flex_kernel, 32 * kFlexWarps, smem),
+                   "flex occupancy");
         const int cols = col_end - col_begin;
-        int blocks = (cols + warps - 1) / warps;
-        blocks = std::max(1, std::min(blocks, sm_count() * 8));
+        const int blocks = std::max(1, std::min(cols, sm_count() * (in_smem ? std::max(per_sm, 1) : 1)));
+        if (!in_smem && blocks * block_doubles > s->scratch_doubles) {
+            if (s->scratch) cudaFree(s->scratch);
+            s->scratch = nullptr;
+            s->scratch_doubles = 0;
+            cuda_check(cudaMalloc(&s->scratch, blocks * block_doubles * sizeof(double)), "cudaMalloc");
+            s->scratch_doubles = blocks * block_doubles;
+        }
+        A.scratch = in_smem ? nullptr : s->scratch;
         if (cols > 0) {
-            flex_kernel<<<blocks, 32 * warps, smem, st>>>(A);
+            flex_kernel<<<blocks, 32 * kFlexWarps, smem, st>>>(A);
             cuda_check(cudaGetLastError(), "flex launch");
         }
         if (tmp_out)

@@ -94,3 +94,39 @@ def test_gpu_full_scan_matches_oracle():
     assert same.mean() >= 0.95
     assert np.abs(pts["tip"] - want["tip"]).max(axis=1)[same].max() < 1e-6
     assert st.total_steps > 0
+
+
+def _with_hydrogens(tmp_path, n_h2, **opt):
+    """The flexible naphthalene with n_h2 more H2 molecules around it."""
+    from mechafm_gb300 import synth
+    spec = synth.flexible_naphthalene(area=0.5, step=0.5, zhigh=10.0, zlow=9.7, dz=0.2, **opt)
+    extra, side = [], int(np.ceil(np.sqrt(n_h2 + 9)))
+    for m in range(side * side):
+        x, y = 5.0 * (m % side - side // 2), 5.0 * (m // side - side // 2)
+        if abs(x) > 7.0 or abs(y) > 4.0:
+            extra += [[x, y - 0.37, 0.2], [x, y + 0.37, 0.2]]
+    extra = extra[:2 * n_h2]
+    spec.types = spec.types + ["H"] * len(extra)
+    spec.pos = np.vstack([spec.pos] + ([extra] if extra else []))
+    spec.charges = np.concatenate([spec.charges, 0.05 * np.tile([1.0, -1.0], len(extra) // 2)])
+    spec.fixed = np.concatenate([spec.fixed, np.zeros(len(extra), dtype=int)])
+    inp = Input(spec.write(str(tmp_path)))
+    return inp, inp.desc(), inp.flex_desc()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_h2,opt", [
+    (0, dict(integrator="euler")), (0, dict(minimiser="SD", dt="0.0005")),   # every path of a step
+    (6, {}),          # 32 atoms and the tip and dummy: more than a warp of atoms
+    (30, {}),         # 80 atoms: more values than the mixing warps have threads
+    (45, dict(integrator="rk4")), (60, {})])   # around where the force slots leave shared memory
+def test_gpu_sizes_match_oracle(tmp_path, n_h2, opt):
+    inp, desc, flex = _with_hydrogens(tmp_path, n_h2, maxsteps="60", **opt)
+    pts, _, states = FlexScan(desc, flex, device=0).run(state_column=1)
+    want, _, _ = oracle.flex_run(desc, flex)
+    _, _, want_states = oracle.flex_run(desc, flex, 1, 2, state_column=1)
+    np.testing.assert_array_equal(pts["steps"], want["steps"])
+    # the bars of the fixtures above: to rounding, carried through 60 steps
+    np.testing.assert_allclose(pts["tip"], want["tip"], rtol=0, atol=1e-6)
+    np.testing.assert_allclose(pts["force"], want["force"], rtol=1e-6, atol=1e-9)
+    np.testing.assert_allclose(states, want_states, rtol=0, atol=1e-6)
