@@ -283,7 +283,7 @@ int mafm_run(mafm_scan* scan, const mafm_run_opts* opts, mafm_point* out,
 /* Relax chosen pixel columns of a scan in plain FP64: for pixels (i, j)
  * given as columns[m] = i*ny + j, in any order and from anywhere in the scan,
  * out[m*nz + k] receives height k (n*nz records, host or device memory, as
- * for mafm_run).  One warp relaxes one column and adds every sum in the
+ * for mafm_run).  Every sum is added in the
  * reference's order, so the points are bit-identical to mafm_run's MAFM_FP64
  * points.  The pixel loop of Simulation::run (simulation.cpp:78-122) over a
  * sample of pixels: used to check a fast run against FP64 on pixels spread

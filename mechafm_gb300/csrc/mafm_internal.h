@@ -164,8 +164,12 @@ struct RunCounters {
 
 // Launchers implemented in relax64.cu / relax32.cu.  ctr points to zeroed
 // device counters owned by the caller.
-cudaError_t launch_relax64(const ScanParams& p, mafm_point* out, RunCounters* ctr,
-                           int col_begin, int col_end, cudaStream_t s);
+// launch_relax64: list (may be null) gives the columns, else col_begin,
+// col_begin + 1, ...; n_cols of them.  by_column: the points of column c go to
+// out + (c - col_begin) nz, else those of the i-th to out + i nz.
+cudaError_t launch_relax64(const ScanParams& p, mafm_point* out, RunCounters* ctr, const int* list,
+                           int col_begin, long long n_cols, int pairs_per_eval, bool by_column,
+                           cudaStream_t s);
 cudaError_t launch_sample64(const ScanParams& p, int what, const double* pts, int64_t n,
                             double* out, RunCounters* ctr, cudaStream_t s);
 cudaError_t launch_grid_build64(const ScanParams& p, const GridView& g, Node64* out,
@@ -199,15 +203,12 @@ cudaError_t launch_relax32(const BatchScan* scans_dev, int n_scans, long long n_
                            const Relax32Config& cfg, RunCounters* ctr, cudaStream_t s);
 // Fills share_begin and weight of a launch's scans.
 void set_batch_shares(BatchScan* scans, int n_scans);
-// FP64 re-relaxation of listed columns (relax64.cu): list[i] = scan index << 32
-// | column for i < min(count, cap), where count = ctr->n_tie when n_fixed < 0
-// (the columns the double-float kernel flagged) and n_fixed otherwise.
-// replace = true marks the points MAFM_PT_FP64 and corrects the step total
-// for the records it overwrites.  The points of column c go to
-// out + (c - col_begin) nz, or with list_out to out + i nz for list entry i.
+// FP64 re-relaxation of the columns the double-float kernel listed (relax64.cu):
+// list[i] = scan index << 32 | column for i < min(ctr->n_tie, cap).  Marks the
+// points MAFM_PT_FP64 and corrects the step total for the records it
+// overwrites.
 cudaError_t launch_repair64(const BatchScan* scans, const unsigned long long* list, unsigned cap,
-                            long long n_fixed, bool replace, bool list_out, RunCounters* ctr,
-                            cudaStream_t s);
+                            RunCounters* ctr, cudaStream_t s);
 cudaError_t launch_sample32(const ScanParams& p, int what, const double* pts, int64_t n,
                             double* out, RunCounters* ctr, cudaStream_t s);
 cudaError_t launch_grid_build32(const ScanParams& p, const GridView& g, float4* out,

@@ -916,7 +916,8 @@ int mafm_run(mafm_scan* scan, const mafm_run_opts* opts, mafm_point* out, mafm_r
         cuda_check(cudaEventRecord(scan->ev0, st), "cudaEventRecord");
         if (prec == MAFM_FP64) {
             ScanParams p = build_params(*scan);
-            cuda_check(launch_relax64(p, dout, scan->ctr.p, cb, ce, st), "relax64 launch");
+            cuda_check(launch_relax64(p, dout, scan->ctr.p, nullptr, cb, ce - cb, scan->n_pairs_per_eval, true, st),
+                       "relax64 launch");
         } else if (prec == MAFM_DF) {
             // double-float relaxation, then FP64 for the columns it lists
             BatchScan b{};
@@ -935,7 +936,7 @@ int mafm_run(mafm_scan* scan, const mafm_run_opts* opts, mafm_point* out, mafm_r
             cuda_check(launch_relaxdf(scan->batchdf.p, scan->batch.p, 1, ce - cb, scan->ctr.p, scan->repair.p, cap,
                                       watchdog_ns_from_env(), opts ? opts->lanes_per_column : 0, st),
                        "double-float relax launch");
-            cuda_check(launch_repair64(scan->batch.p, scan->repair.p, cap, -1, true, false, scan->ctr.p, st),
+            cuda_check(launch_repair64(scan->batch.p, scan->repair.p, cap, scan->ctr.p, st),
                        "FP64 re-relaxation launch");
         } else {
             BatchScan b{};
@@ -1060,7 +1061,7 @@ int mafm_run_batch(mafm_scan* const* scans, int32_t n_scans, const mafm_run_opts
             cuda_check(launch_relaxdf(dbd.p, dbs.p, n_scans, total_cols, s0->ctr.p, rlist.p, (unsigned)total_cols,
                                       watchdog_ns_from_env(), opts ? opts->lanes_per_column : 0, st),
                        "double-float relax launch");
-            cuda_check(launch_repair64(dbs.p, rlist.p, (unsigned)total_cols, -1, true, false, s0->ctr.p, st),
+            cuda_check(launch_repair64(dbs.p, rlist.p, (unsigned)total_cols, s0->ctr.p, st),
                        "FP64 re-relaxation launch");
         } else {
             cuda_check(launch_relax32(dbs.p, n_scans, total_cols, next_col.p, cfg, s0->ctr.p, st),
@@ -1101,12 +1102,9 @@ int mafm_run_columns(mafm_scan* scan, const int32_t* columns, int64_t n, mafm_po
         if (n == 0) return;
         const long long n_cols = (long long)scan->d.nx * scan->d.ny;
         if (n > 0xffffffffll) fail(MAFM_E_RANGE, "more than 2^32 columns in one call");
-        std::vector<unsigned long long> list((size_t)n);
-        for (int64_t i = 0; i < n; ++i) {
+        for (int64_t i = 0; i < n; ++i)
             if (columns[i] < 0 || columns[i] >= n_cols)
                 fail(MAFM_E_INVALID, "column %d outside [0, %lld)", columns[i], n_cols);
-            list[(size_t)i] = (unsigned long long)(unsigned)columns[i];
-        }
         cuda_check(cudaSetDevice(scan->device), "cudaSetDevice");
         cudaStream_t st = (cudaStream_t)stream;
         const size_t n_pts = (size_t)n * scan->d.nz;
@@ -1119,23 +1117,14 @@ int mafm_run_columns(mafm_scan* scan, const int32_t* columns, int64_t n, mafm_po
             dout = scan->stage.p;
         }
         ensure_grid(*scan, true, st);
-        DevBuf<unsigned long long> dlist;
+        DevBuf<int> dlist;
         dlist.alloc((size_t)n);
-        cuda_check(cudaMemcpyAsync(dlist.p, list.data(), (size_t)n * sizeof(unsigned long long),
-                                   cudaMemcpyHostToDevice, st), "upload columns");
-        BatchScan b{};
-        b.p = build_params(*scan);
-        b.out = dout;
-        b.col_begin = 0;
-        b.col_end = (int)n_cols;
-        b.n_pairs_per_eval = scan->n_pairs_per_eval;
-        b.has_coulomb = scan->has_coulomb;
-        write_batch<<<1, 1, 0, st>>>(scan->batch.p, b);
-        cuda_check(cudaGetLastError(), "descriptor upload");
+        cuda_check(cudaMemcpyAsync(dlist.p, columns, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, st),
+                   "upload columns");
         zero_counters(*scan, st);
         cuda_check(cudaEventRecord(scan->ev0, st), "cudaEventRecord");
-        cuda_check(launch_repair64(scan->batch.p, dlist.p, (unsigned)n, n, false, true, scan->ctr.p, st),
-                   "FP64 column launch");
+        cuda_check(launch_relax64(build_params(*scan), dout, scan->ctr.p, dlist.p, 0, n, scan->n_pairs_per_eval,
+                                  false, st), "FP64 column launch");
         cuda_check(cudaEventRecord(scan->ev1, st), "cudaEventRecord");
         if (staged)
             cuda_check(cudaMemcpyAsync(out, dout, n_pts * sizeof(mafm_point), cudaMemcpyDeviceToHost, st),
@@ -1363,7 +1352,7 @@ void plan_launch(mafm_plan& p, cudaStream_t st) {
         cuda_check(launch_relaxdf(p.listdf.p, p.list.p, p.n_scans, p.cols, p.ctr.p, p.repair.p,
                                   (unsigned)p.cols, p.cfg.watchdog_ns, p.df_lanes, st),
                    "double-float relax launch");
-        cuda_check(launch_repair64(p.list.p, p.repair.p, (unsigned)p.cols, -1, true, false, p.ctr.p, st),
+        cuda_check(launch_repair64(p.list.p, p.repair.p, (unsigned)p.cols, p.ctr.p, st),
                    "FP64 re-relaxation launch");
     } else {
         cuda_check(launch_relax32(p.list.p, p.n_scans, p.cols, p.next_col.p, p.cfg, p.ctr.p, st), "relax32 launch");
