@@ -67,6 +67,7 @@ struct ScanParamsDF {
     dfloat dx, dy, dz, zhigh;
     dfloat cell[9], cell_inv[9], offset[3];
     int minimiser, integrator, minterm, maxsteps;
+    unsigned stage_mask;   // evaluations per step - 1
     dfloat etol, ftol, dt;
     TieMargins tie;
 };

@@ -546,9 +546,17 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
             break;
         }
         if (s.col < 0) continue;
+        const ScanParamsDF& P = B->p;
+        // A step starts, and a height's record is made, only in every second
+        // iteration (midpoint; rk4: every fourth), so that the lanes of a warp
+        // are in the same stage: without it they drift apart by one evaluation
+        // at every record, and the warp runs every stage's code in every
+        // iteration.  A lane waits for at most one (three) of a height's
+        // hundreds of evaluations (401 x 401 cluster 627 -> 599 ms, 101 x 101
+        // graphene 115 -> 107 ms).
+        if ((s.phase == DF_EVAL0 || s.phase == DF_OUT) && (ticks & P.stage_mask)) continue;
 
         // ---- one evaluation per lane ----
-        const ScanParamsDF& P = B->p;
         V3D F;
         D E;
         ts_df<G>(P, s.ex, sub, gmask, F, E, s.outside, err);
@@ -916,6 +924,8 @@ ScanParamsDF params_df(const ScanParams& p, const TermPairDF* pairs, int n_lj_pa
     q.dx = D(p.dx); q.dy = D(p.dy); q.dz = D(p.dz); q.zhigh = D(p.zhigh);
     q.minimiser = p.minimiser;
     q.integrator = p.integrator;
+    q.stage_mask = p.minimiser == MAFM_MIN_SD || p.integrator == MAFM_INT_EULER ? 0u
+                   : p.integrator == MAFM_INT_MIDPOINT ? 1u : 3u;
     q.minterm = p.minterm;
     q.maxsteps = p.maxsteps;
     q.etol = D(p.etol);
