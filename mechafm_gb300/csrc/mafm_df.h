@@ -104,12 +104,46 @@ cudaError_t launch_relaxdf(const BatchDF* scans, const BatchScan* scans64, int n
 int df_lanes_per_column(long long n_cols, int requested);
 // The external field's FP64 nodes as double-float.
 cudaError_t launch_nodes_to_df(const Node64* in, NodeDF* out, long long n, cudaStream_t s);
+// ---- the rigid grid's build with interpolated far terms (relaxdf.cu) ----
+constexpr int kFarPoints = 16;       // Chebyshev points per axis and block
+constexpr int kFarMaxNodes = 40;     // nodes per axis and block
+// Half axis of the smallest ellipse of analyticity a far term has on every axis
+// (the block's interval being [-1, 1]): 10 means a convergence rate of 20 per point.
+constexpr float kFarAxis = 10.0f;
+
+// One axis of a plan: block b holds nodes begin[b] .. begin[b + 1] - 1.
+struct FarAxisDF {
+    std::vector<int> begin;
+    std::vector<dfloat> pos;         // of every node (wrapped)
+    std::vector<dfloat> cheb;        // kFarPoints per block
+    std::vector<dfloat> lag;         // kFarPoints weights per node
+    std::vector<float2> box;         // centre and half size of every block
+};
+struct FarPlanDF {
+    FarAxisDF axis[3];
+    int words = 0;                   // of a block's near mask
+};
+// The same on the device, with its workspaces.
+struct FarViewDF {
+    int nb[3];
+    const int* begin[3];
+    const dfloat* pos[3];
+    const dfloat* cheb[3];
+    const dfloat* lag[3];
+    const float2* box[3];
+    int words, max_strips, max_planes;
+    unsigned* mask;                  // words per block
+    NodeDF* coef;                    // kFarPoints^3 per block
+};
+bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float>& xyz, FarPlanDF& plan);
+
 // Simulation::buildTipGridInteractions (simulation.cpp:420-501) in
 // double-float: the rigid grid of geometry p.grid (p.ts_mode 0 or 1: the
 // terms, and the external field) into out, then its FP64 copy (each node's
 // h + l, exact in FP64) into out64 for the FP64 re-relaxation; device error
-// bits (a lookup of the external field) are ORed into *err_word.
+// bits (a lookup of the external field) are ORed into *err_word.  far: the plan
+// of the interpolated build, null for every term at every node.
 cudaError_t launch_grid_builddf(const ScanParamsDF& p, NodeDF* out, Node64* out64, unsigned* err_word,
-                                cudaStream_t s);
+                                const FarViewDF* far, cudaStream_t s);
 
 }  // namespace mafm

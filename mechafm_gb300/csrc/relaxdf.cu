@@ -34,6 +34,7 @@
 // external field lookup force_grid.cpp:88-275, minimiser and column as in
 // relax_tpl.cuh.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 
 #include "mafm_df.h"
@@ -772,6 +773,30 @@ __global__ void nodes_to_df_kernel(const Node64* in, NodeDF* out, long long n) {
     }
 }
 
+// The sums of the NB tips of a strip (the same x and y).
+template <int NB>
+struct StripSums {
+    LazySum2 fx[NB], fy[NB], fz[NB], ee[NB];
+};
+
+// One record for a strip: the x and y separations and their squares once for all
+// of its tips.
+template <int NB>
+__device__ __forceinline__ void strip_record(const ScanParamsDF& p, int r, D2 tx, D2 ty, const D2 (&tz)[NB],
+                                             StripSums<NB>& sm) {
+    const bool lj = r < p.n_lj_pairs;
+    const PairDF2 t = lj ? load_pair<MAFM_PAIR_LJ>(p.pairs + r) : load_pair<MAFM_PAIR_MORSE>(p.pairs + r);
+    const D2 dx = dfl2_sub_u(tx, t.x), dy = dfl2_sub_u(ty, t.y);
+    const D2 dxy2 = dfl2_add_u(sq_u(dx), sq_u(dy));
+#pragma unroll
+    for (int m = 0; m < NB; ++m) {
+        const D2 dz = dfl2_sub_u(tz[m], t.z);
+        const D2 r2 = dfl2_add_u(dxy2, sq_u(dz));
+        if (lj) pair_df2_at<MAFM_PAIR_LJ>(t, dx, dy, dz, r2, sm.fx[m], sm.fy[m], sm.fz[m], sm.ee[m]);
+        else pair_df2_at<MAFM_PAIR_MORSE>(t, dx, dy, dz, r2, sm.fx[m], sm.fy[m], sm.fz[m], sm.ee[m]);
+    }
+}
+
 // Simulation::buildTipGridInteractions (simulation.cpp:420-501) in
 // double-float.  One thread per strip of NB consecutive nodes of a grid
 // column (z fastest, so a warp's strips share x and y and read the same term
@@ -785,7 +810,7 @@ __global__ void __launch_bounds__(128) grid_builddf_kernel(const ScanParamsDF p,
     const GridViewDF& g = p.grid;
     const int nzs = (g.n[2] + NB - 1) / NB;
     const long long total = (long long)g.n[0] * g.n[1] * nzs;
-    const int n_lj = p.n_lj_pairs, n_all = p.n_lj_pairs + p.n_morse_pairs;
+    const int n_all = p.n_lj_pairs + p.n_morse_pairs;
     unsigned err = 0;
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
@@ -799,26 +824,14 @@ __global__ void __launch_bounds__(128) grid_builddf_kernel(const ScanParamsDF p,
         D2 tz[NB];
 #pragma unroll
         for (int m = 0; m < NB; ++m) tz[m] = dfl2(D(k0 + m) * g.basis[8] + g.origin[2]);
-        LazySum2 fx[NB], fy[NB], fz[NB], ee[NB];
+        StripSums<NB> sm;
 #pragma unroll 1
-        for (int r = 0; r < n_all; ++r) {
-            const bool lj = r < n_lj;
-            const PairDF2 t = lj ? load_pair<MAFM_PAIR_LJ>(p.pairs + r) : load_pair<MAFM_PAIR_MORSE>(p.pairs + r);
-            const D2 dx = dfl2_sub_u(tx, t.x), dy = dfl2_sub_u(ty, t.y);
-            const D2 dxy2 = dfl2_add_u(sq_u(dx), sq_u(dy));
-#pragma unroll
-            for (int m = 0; m < NB; ++m) {
-                const D2 dz = dfl2_sub_u(tz[m], t.z);
-                const D2 r2 = dfl2_add_u(dxy2, sq_u(dz));
-                if (lj) pair_df2_at<MAFM_PAIR_LJ>(t, dx, dy, dz, r2, fx[m], fy[m], fz[m], ee[m]);
-                else pair_df2_at<MAFM_PAIR_MORSE>(t, dx, dy, dz, r2, fx[m], fy[m], fz[m], ee[m]);
-            }
-        }
+        for (int r = 0; r < n_all; ++r) strip_record<NB>(p, r, tx, ty, tz, sm);
 #pragma unroll
         for (int m = 0; m < NB; ++m) {
             if (k0 + m >= g.n[2]) break;
-            V3D F = {fx[m].value(), fy[m].value(), fz[m].value()};
-            D E = ee[m].value();
+            V3D F = {sm.fx[m].value(), sm.fy[m].value(), sm.fz[m].value()};
+            D E = sm.ee[m].value();
             if (p.ts_mode == 1) {
                 V3D f;
                 D e;
@@ -838,6 +851,197 @@ __global__ void nodes_df_to_64_kernel(const NodeDF* in, Node64* out, long long n
          i += (long long)gridDim.x * blockDim.x) {
         const NodeDF v = in[i];
         out[i] = Node64{to_double(v.x), to_double(v.y), to_double(v.z), to_double(v.w)};
+    }
+}
+
+// ---- grid build with interpolated far terms -------------------------------------
+//
+// Far from an atom its force is smooth, so within a block of nodes the sum over
+// the far records is evaluated at 16 x 16 x 16 Chebyshev points and interpolated
+// to the block's nodes, and only the records near the block are evaluated at every
+// node.  A record is far from a block when, on every axis, the ellipse around the
+// block's interval (scaled to [-1, 1]) on which the term has its nearest
+// singularity has a half axis of at least kFarAxis: a term (r^-1 to r^-14) is then
+// interpolated to 1e-15 of itself or better (the r^-14 part, which converges
+// slowest, is below 1e-4 of its r^-7 part there).  Blocks, Chebyshev points and
+// the interpolation weights are laid out once (plan_far_df); every build
+// classifies the records and evaluates all of it.
+//
+// Slab of 9,216 records: 64 x 64 px (157 x 157 x 141 nodes) 270 -> 46 ms, 256 x 256
+// px (541 x 541 x 141) 3198 -> 479 ms; and fewer roundings per node: the relaxed
+// forces' error against FP64 falls from 3e-13 to 1e-14.
+
+constexpr int kFarP = kFarPoints;
+
+// Half axis of the ellipse through a singularity at distance off along the axis
+// from the interval's centre and gap beside it.
+__host__ __device__ __forceinline__ float far_axis(float off, float gap, float half) {
+    const float u = off / half, v = gap / half;
+    return 0.5f * (sqrtf((u - 1) * (u - 1) + v * v) + sqrtf((u + 1) * (u + 1) + v * v));
+}
+
+// Whether the point a is near the box of centre c and half sizes h.
+__host__ __device__ __forceinline__ bool near_box(const float a[3], const float c[3], const float h[3]) {
+    float d[3], gap[3];
+    for (int m = 0; m < 3; ++m) {
+        d[m] = fabsf(a[m] - c[m]);
+        gap[m] = fmaxf(d[m] - h[m], 0.f);
+    }
+    for (int m = 0; m < 3; ++m) {
+        const float ga = gap[(m + 1) % 3], gb = gap[(m + 2) % 3];
+        if (far_axis(d[m], sqrtf(ga * ga + gb * gb), h[m]) < kFarAxis) return true;
+    }
+    return false;
+}
+
+struct FarBlock {
+    int b[3];        // block index per axis
+};
+
+__device__ __forceinline__ FarBlock far_block(const FarViewDF& f, int id) {
+    FarBlock q;
+    q.b[2] = id % f.nb[2];
+    q.b[1] = id / f.nb[2] % f.nb[1];
+    q.b[0] = id / f.nb[2] / f.nb[1];
+    return q;
+}
+
+// One bit per record and block: set when either of its terms is near.
+__global__ void far_classify_kernel(const FarViewDF f, const TermPairDF* pairs, int n_rec) {
+    const FarBlock q = far_block(f, blockIdx.x);
+    float c[3], h[3];
+    for (int a = 0; a < 3; ++a) {
+        c[a] = f.box[a][q.b[a]].x;
+        h[a] = f.box[a][q.b[a]].y;
+    }
+    for (int w = threadIdx.x; w < f.words; w += blockDim.x) {
+        unsigned bits = 0;
+        for (int k = 0; k < 32 && 32 * w + k < n_rec; ++k) {
+            const TermPairDF& t = pairs[32 * w + k];
+            const float a0[3] = {t.xh.x, t.yh.x, t.zh.x}, a1[3] = {t.xh.y, t.yh.y, t.zh.y};
+            if (near_box(a0, c, h) || near_box(a1, c, h)) bits |= 1u << k;
+        }
+        f.mask[(size_t)blockIdx.x * f.words + w] = bits;
+    }
+}
+
+// The near (or the far) records of a block for a strip, and the strip's values.
+// The words are the same for all threads of the block: no divergence.
+template <int NB>
+__device__ __forceinline__ void strip_masked(const ScanParamsDF& p, const unsigned* mask, int words, bool far,
+                                             D x, D y, const D (&z)[NB], NodeDF (&val)[NB]) {
+    const D2 tx = dfl2(x), ty = dfl2(y);
+    D2 tz[NB];
+#pragma unroll
+    for (int m = 0; m < NB; ++m) tz[m] = dfl2(z[m]);
+    StripSums<NB> sm;
+    const int n_rec = p.n_lj_pairs + p.n_morse_pairs;
+    for (int w = 0; w < words; ++w) {
+        unsigned bits = __ldg(mask + w);
+        if (far) bits = ~bits & (n_rec - 32 * w >= 32 ? 0xffffffffu : (1u << (n_rec - 32 * w)) - 1u);
+#pragma unroll 1
+        while (bits) {
+            const int r = 32 * w + __ffs(bits) - 1;
+            bits &= bits - 1;
+            strip_record<NB>(p, r, tx, ty, tz, sm);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < NB; ++m)
+        val[m] = NodeDF{sm.fx[m].value(), sm.fy[m].value(), sm.fz[m].value(), sm.ee[m].value()};
+}
+
+// The far sums at a block's Chebyshev points: blockIdx.y the block, a thread four
+// points along z.
+__global__ void __launch_bounds__(128) far_coef_kernel(const ScanParamsDF p, const FarViewDF f) {
+    const FarBlock q = far_block(f, blockIdx.y);
+    const int t = blockIdx.x * 128 + threadIdx.x;   // < kFarP * kFarP * kFarP / 4
+    const int k0 = t % (kFarP / 4) * 4, j = t / (kFarP / 4) % kFarP, i = t / (kFarP / 4) / kFarP;
+    D z[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) z[m] = f.cheb[2][q.b[2] * kFarP + k0 + m];
+    NodeDF val[4];
+    strip_masked<4>(p, f.mask + (size_t)blockIdx.y * f.words, f.words, true,
+                                f.cheb[0][q.b[0] * kFarP + i], f.cheb[1][q.b[1] * kFarP + j], z, val);
+    NodeDF* o = f.coef + ((size_t)blockIdx.y * kFarP * kFarP + i * kFarP + j) * kFarP + k0;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) o[m] = val[m];
+}
+
+// The near sums at a block's nodes, a thread four nodes along z.
+__global__ void __launch_bounds__(128) far_near_kernel(const ScanParamsDF p, const FarViewDF f, NodeDF* out) {
+    const FarBlock q = far_block(f, blockIdx.y);
+    int lo[3], n[3];
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = f.begin[a][q.b[a]];
+        n[a] = f.begin[a][q.b[a] + 1] - lo[a];
+    }
+    const int nzs = (n[2] + 3) / 4;
+    const int t = blockIdx.x * 128 + threadIdx.x;
+    if (t >= n[0] * n[1] * nzs) return;
+    const int k0 = lo[2] + t % nzs * 4, j = lo[1] + t / nzs % n[1], i = lo[0] + t / nzs / n[1];
+    const int k1 = lo[2] + n[2];
+    D z[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) z[m] = f.pos[2][min(k0 + m, k1 - 1)];
+    NodeDF val[4];
+    strip_masked<4>(p, f.mask + (size_t)blockIdx.y * f.words, f.words, false, f.pos[0][i], f.pos[1][j],
+                                z, val);
+    NodeDF* o = out + ((long long)i * p.grid.n[1] + j) * p.grid.n[2];
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+        if (k0 + m < k1) o[k0 + m] = val[m];
+}
+
+// sum_m l[m] c[m stride] of the nodes' four values, two per packed operation.
+__device__ __forceinline__ NodeDF far_dot(const D* l, const NodeDF* c, int stride) {
+    D2 f0 = {p_bcast(0.f), p_bcast(0.f)}, f1 = f0;
+#pragma unroll 4
+    for (int m = 0; m < kFarP; ++m) {
+        const float4* v = reinterpret_cast<const float4*>(c + m * stride);
+        const float4 a = v[0], b = v[1];
+        const D2 w = dfl2(l[m]);
+        f0 = dfl2_add_u(f0, dfl2_mul_u(D2{make_float2(a.x, a.z), make_float2(a.y, a.w)}, w));
+        f1 = dfl2_add_u(f1, dfl2_mul_u(D2{make_float2(b.x, b.z), make_float2(b.y, b.w)}, w));
+    }
+    f0 = dfl2_norm(f0);
+    f1 = dfl2_norm(f1);
+    return NodeDF{dfl2_x(f0), dfl2_y(f0), dfl2_x(f1), dfl2_y(f1)};
+}
+
+// The far sums interpolated to a plane of a block's nodes (blockIdx.x: the plane
+// along x, blockIdx.y: the block), added to the near sums in out, with the
+// external field (ts_mode 1); and the nodes' FP64 copy.
+__global__ void __launch_bounds__(256) far_interp_kernel(const ScanParamsDF p, const FarViewDF f, NodeDF* out,
+                                                         Node64* out64) {
+    __shared__ NodeDF plane[kFarP * kFarP];              // at the node's x
+    __shared__ NodeDF rows[kFarMaxNodes * kFarP];        // at the nodes' x, y
+    const FarBlock q = far_block(f, blockIdx.y);
+    const int i = f.begin[0][q.b[0]] + blockIdx.x;
+    if (i >= f.begin[0][q.b[0] + 1]) return;
+    const int j0 = f.begin[1][q.b[1]], ny = f.begin[1][q.b[1] + 1] - j0;
+    const int k0 = f.begin[2][q.b[2]], nz = f.begin[2][q.b[2] + 1] - k0;
+    const NodeDF* c = f.coef + (size_t)blockIdx.y * kFarP * kFarP * kFarP;
+    for (int t = threadIdx.x; t < kFarP * kFarP; t += 256)
+        plane[t] = far_dot(f.lag[0] + i * kFarP, c + t, kFarP * kFarP);
+    __syncthreads();
+    for (int t = threadIdx.x; t < ny * kFarP; t += 256)
+        rows[t] = far_dot(f.lag[1] + (j0 + t / kFarP) * kFarP, plane + t % kFarP, kFarP);
+    __syncthreads();
+    for (int t = threadIdx.x; t < ny * nz; t += 256) {
+        const int j = t / nz, k = t % nz;
+        const NodeDF v = far_dot(f.lag[2] + (k0 + k) * kFarP, rows + j * kFarP, 1);
+        const long long at = ((long long)i * p.grid.n[1] + j0 + j) * p.grid.n[2] + k0 + k;
+        const NodeDF nr = out[at];
+        NodeDF s = {nr.x + v.x, nr.y + v.y, nr.z + v.z, nr.w + v.w};
+        if (p.ts_mode == 1) {
+            V3D fe;
+            D e;
+            interp_df(p.es, V3D{f.pos[0][i], f.pos[1][j0 + j], f.pos[2][k0 + k]}, fe, e);
+            s = {s.x + fe.x, s.y + fe.y, s.z + fe.z, s.w + e};
+        }
+        out[at] = s;
+        out64[at] = Node64{to_double(s.x), to_double(s.y), to_double(s.z), to_double(s.w)};
     }
 }
 
@@ -1016,10 +1220,146 @@ cudaError_t launch_nodes_to_df(const Node64* in, NodeDF* out, long long n, cudaS
     return cudaGetLastError();
 }
 
+// Lay out the blocks of a rigid grid for the interpolated build, or return false
+// where it would not pay: the node positions (x and y wrapped into the cell, on
+// the host as the FP64 build wraps them), blocks of about the length that costs
+// least by the estimate below, none across a jump of the wrapped positions, and
+// for every axis Chebyshev points and the weights of the block's nodes.  xyz: the
+// positions of the records' two terms.
+bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float>& xyz, FarPlanDF& plan) {
+    const long long n_rec = (long long)xyz.size() / 6;
+    if (n_rec < 64) return false;
+    if (p.tip_pbc)
+        for (int r = 0; r < 3; ++r)
+            for (int c = 0; c < 3; ++c)
+                if (r != c && (p.cell[3 * r + c] != 0 || p.cell_inv[3 * r + c] != 0)) return false;
+    std::vector<double> pos[3];
+    for (int a = 0; a < 3; ++a) {
+        pos[a].resize(g.n[a]);
+        for (int i = 0; i < g.n[a]; ++i) {
+            double x = i * g.basis[4 * a] + g.origin[a];
+            if (p.tip_pbc && a < 2) {   // System::setDummyXY for a diagonal cell
+                double cn = p.cell_inv[4 * a] * (x - p.offset[a]);
+                cn -= std::floor(cn);
+                x = p.cell[4 * a] * cn + p.offset[a];
+            }
+            pos[a][i] = x;
+        }
+    }
+    // blocks of one axis: runs without a jump, cut evenly to at most length len
+    auto cut = [&](int a, double len) {
+        const double s = g.basis[4 * a];
+        const int most = std::min(std::max((int)(len / s + 0.5) + 1, 2), kFarMaxNodes);
+        std::vector<int> begin;
+        for (int i = 0; i < g.n[a];) {
+            int e = i + 1;
+            while (e < g.n[a] && std::fabs(pos[a][e] - pos[a][e - 1] - s) < 0.01 * s) ++e;
+            const int parts = (e - i + most - 1) / most;
+            for (int q = 0; q < parts; ++q) begin.push_back(i + (int)((long long)(e - i) * q / parts));
+            i = e;
+        }
+        begin.push_back(g.n[a]);
+        return begin;
+    };
+    auto box = [&](int a, const std::vector<int>& begin, int b) {
+        const double lo = pos[a][begin[b]], hi = pos[a][begin[b + 1] - 1];
+        // one node: an interval around it
+        return std::make_pair(0.5 * (lo + hi), std::max(0.5 * (hi - lo), 0.5 * g.basis[4 * a]));
+    };
+    const double nodes = (double)g.n[0] * g.n[1] * g.n[2];
+    const double direct = nodes * n_rec;
+    const long long step = (n_rec + 1023) / 1024;
+    double best = 0.7 * direct;
+    std::vector<int> begin[3];
+    for (double len : {1.6, 2.4, 3.2, 4.8, 6.4}) {
+        std::vector<int> bg[3];
+        double blocks = 1;
+        for (int a = 0; a < 3; ++a) {
+            bg[a] = cut(a, len);
+            blocks *= (double)bg[a].size() - 1;
+        }
+        const double coef = blocks * kFarP * kFarP * kFarP;
+        if (blocks > 65535 || coef * sizeof(NodeDF) > 8e9 || coef * n_rec > best) continue;
+        // near records, of a few blocks and at most about 1,000 records
+        double near = 0;
+        long long tried = 0;
+        for (int q : {0, 7, 8}) {   // two corners and the middle
+            float c[3], h[3];
+            for (int a = 0; a < 3; ++a) {
+                const int last = (int)bg[a].size() - 2;
+                const auto b = box(a, bg[a], q == 8 ? last / 2 : (q >> a & 1) ? last : 0);
+                c[a] = (float)b.first;
+                h[a] = (float)b.second;
+            }
+            for (long long r = 0; r < n_rec; r += step, ++tried)
+                near += near_box(&xyz[6 * r], c, h) || near_box(&xyz[6 * r + 3], c, h);
+        }
+        near *= (double)n_rec / tried;
+        // per node the interpolation costs about four records
+        const double cost = coef * (n_rec - near) + nodes * (near + 4);
+        if (cost < best) {
+            best = cost;
+            for (int a = 0; a < 3; ++a) begin[a] = bg[a];
+        }
+    }
+    if (begin[0].empty()) return false;
+    const double pi = 3.14159265358979323846;
+    for (int a = 0; a < 3; ++a) {
+        FarAxisDF& A = plan.axis[a];
+        A.begin = begin[a];
+        A.pos.clear();
+        for (double x : pos[a]) A.pos.push_back(D(x));
+        A.lag.assign((size_t)g.n[a] * kFarP, D(0.0f, 0.0f));
+        A.cheb.clear();
+        A.box.clear();
+        for (size_t b = 0; b + 1 < begin[a].size(); ++b) {
+            const auto bx = box(a, begin[a], (int)b);
+            A.box.push_back(make_float2((float)bx.first, (float)bx.second));
+            long double x[kFarP], w[kFarP];
+            for (int m = 0; m < kFarP; ++m) {
+                const D q(bx.first + bx.second * std::cos((2 * m + 1) * pi / (2 * kFarP)));
+                A.cheb.push_back(q);
+                x[m] = (long double)q.h + (long double)q.l;   // the point as the kernels have it
+            }
+            for (int m = 0; m < kFarP; ++m) {
+                w[m] = 1;
+                for (int k = 0; k < kFarP; ++k)
+                    if (k != m) w[m] *= 2 * (x[m] - x[k]) / (long double)bx.second;
+                w[m] = 1 / w[m];
+            }
+            for (int i = begin[a][b]; i < begin[a][b + 1]; ++i) {
+                const D q = A.pos[i];
+                const long double v = (long double)q.h + (long double)q.l;
+                long double sum = 0;
+                int hit = -1;
+                for (int m = 0; m < kFarP; ++m) {
+                    if (v == x[m]) hit = m;
+                    else sum += w[m] / (v - x[m]);
+                }
+                for (int m = 0; m < kFarP; ++m)
+                    A.lag[(size_t)i * kFarP + m] =
+                        hit >= 0 ? D(hit == m ? 1.0f : 0.0f, 0.0f) : D((double)(w[m] / (v - x[m]) / sum));
+            }
+        }
+    }
+    plan.words = (int)((n_rec + 31) / 32);
+    return true;
+}
+
+static cudaError_t launch_far(const ScanParamsDF& p, NodeDF* out, Node64* out64, const FarViewDF& f, cudaStream_t s) {
+    const unsigned blocks = (unsigned)((long long)f.nb[0] * f.nb[1] * f.nb[2]);
+    far_classify_kernel<<<blocks, 128, 0, s>>>(f, p.pairs, p.n_lj_pairs + p.n_morse_pairs);
+    far_coef_kernel<<<dim3(kFarP * kFarP * kFarP / 4 / 128, blocks), 128, 0, s>>>(p, f);
+    far_near_kernel<<<dim3((unsigned)((f.max_strips + 127) / 128), blocks), 128, 0, s>>>(p, f, out);
+    far_interp_kernel<<<dim3((unsigned)f.max_planes, blocks), 256, 0, s>>>(p, f, out, out64);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_grid_builddf(const ScanParamsDF& p, NodeDF* out, Node64* out64, unsigned* err_word,
-                                cudaStream_t s) {
+                                const FarViewDF* far, cudaStream_t s) {
     const long long n = (long long)p.grid.n[0] * p.grid.n[1] * p.grid.n[2];
     if (n <= 0) return cudaSuccess;
+    if (far) return launch_far(p, out, out64, *far, s);
     ScanParamsDF q = p;
     q.grid.g = out;
     constexpr int kNB = 4;

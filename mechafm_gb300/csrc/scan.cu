@@ -235,6 +235,13 @@ struct mafm_scan {
     mafm::DevBuf<mafm::NodeDF> griddf;         // rigid grid built in double-float
     mafm::DevBuf<mafm::Node64> griddf64;       //   and its FP64 copy (re-relaxation)
     bool griddf_built = false;
+    // the interpolated build of it: laid out at the first build, where it pays
+    std::vector<float> df_xyz;                 // positions of the term pairs (rigid grids)
+    bool far_planned = false, far_used = false;
+    mafm::FarViewDF far{};
+    mafm::DevBuf<unsigned char> far_tables;
+    mafm::DevBuf<unsigned> far_mask;
+    mafm::DevBuf<mafm::NodeDF> far_coef;
     mafm::DevBuf<mafm::BatchDF> batchdf;       // descriptor of a double-float run
     mafm::DevBuf<unsigned long long> repair;   // columns to re-relax in FP64
     bool order_built = false;
@@ -395,6 +402,9 @@ void pack_terms(mafm_scan& s, const mafm_scan_desc& d) {
     }
     // double-float pairs for MAFM_DF
     const std::vector<TermPairDF> tdf = term_pairs_df(t64, s.df_lj_pairs, s.df_morse_pairs);
+    if (d.rigidgrid)
+        for (const TermPairDF& q : tdf)
+            s.df_xyz.insert(s.df_xyz.end(), {q.xh.x, q.yh.x, q.zh.x, q.xh.y, q.yh.y, q.zh.y});
     s.pairsdf.alloc(std::max<size_t>(tdf.size(), 1));
     if (!tdf.empty())
         cuda_check(cudaMemcpy(s.pairsdf.p, tdf.data(), tdf.size() * sizeof(TermPairDF),
@@ -595,6 +605,57 @@ void ensure_grid(mafm_scan& s, bool fp64, cudaStream_t st, bool rebuild = false)
     s.P.grid = s.grid_view;
 }
 
+// The interpolated build's plan on the device (once per scan).
+void ensure_far_plan(mafm_scan& s, cudaStream_t st) {
+    if (s.far_planned) return;
+    FarPlanDF plan;
+    if (plan_far_df(build_grid_params(s), s.grid_view, s.df_xyz, plan)) {
+        std::vector<unsigned char> host;
+        auto piece = [&](const void* p, size_t bytes) {
+            const size_t at = (host.size() + 63) & ~(size_t)63;
+            host.resize(at + bytes);
+            std::memcpy(host.data() + at, p, bytes);
+            return at;
+        };
+        size_t at[3][5];
+        long long blocks = 1, strips = 1;
+        for (int a = 0; a < 3; ++a) {
+            const FarAxisDF& A = plan.axis[a];
+            at[a][0] = piece(A.begin.data(), A.begin.size() * sizeof(int));
+            at[a][1] = piece(A.pos.data(), A.pos.size() * sizeof(dfloat));
+            at[a][2] = piece(A.cheb.data(), A.cheb.size() * sizeof(dfloat));
+            at[a][3] = piece(A.lag.data(), A.lag.size() * sizeof(dfloat));
+            at[a][4] = piece(A.box.data(), A.box.size() * sizeof(float2));
+            s.far.nb[a] = (int)A.begin.size() - 1;
+            blocks *= s.far.nb[a];
+            int most = 0;
+            for (int b = 0; b < s.far.nb[a]; ++b) most = std::max(most, A.begin[b + 1] - A.begin[b]);
+            if (a == 0) s.far.max_planes = most;
+            strips *= a == 2 ? (most + 3) / 4 : most;
+        }
+        s.far_tables.alloc(host.size());
+        s.far_mask.alloc((size_t)blocks * plan.words);
+        s.far_coef.alloc((size_t)blocks * kFarPoints * kFarPoints * kFarPoints);
+        cuda_check(cudaMemcpyAsync(s.far_tables.p, host.data(), host.size(), cudaMemcpyHostToDevice, st),
+                   "upload grid plan");
+        cuda_check(cudaStreamSynchronize(st), "upload grid plan");
+        for (int a = 0; a < 3; ++a) {
+            const unsigned char* t = s.far_tables.p;
+            s.far.begin[a] = reinterpret_cast<const int*>(t + at[a][0]);
+            s.far.pos[a] = reinterpret_cast<const dfloat*>(t + at[a][1]);
+            s.far.cheb[a] = reinterpret_cast<const dfloat*>(t + at[a][2]);
+            s.far.lag[a] = reinterpret_cast<const dfloat*>(t + at[a][3]);
+            s.far.box[a] = reinterpret_cast<const float2*>(t + at[a][4]);
+        }
+        s.far.words = plan.words;
+        s.far.max_strips = (int)strips;
+        s.far.mask = s.far_mask.p;
+        s.far.coef = s.far_coef.p;
+        s.far_used = true;
+    }
+    s.far_planned = true;
+}
+
 // The double-float rigid grid (MAFM_DF) and its FP64 copy, built on first use
 // (rebuild: again).
 void ensure_grid_df(mafm_scan& s, cudaStream_t st, bool rebuild = false) {
@@ -604,11 +665,13 @@ void ensure_grid_df(mafm_scan& s, cudaStream_t st, bool rebuild = false) {
     const long long N = (long long)s.grid_view.n[0] * s.grid_view.n[1] * s.grid_view.n[2];
     if (!s.griddf.p) s.griddf.alloc((size_t)N);
     if (!s.griddf64.p) s.griddf64.alloc((size_t)N);
+    ensure_far_plan(s, st);
     zero_counters(s, st);
     ScanParams bp = build_grid_params(s);
     bp.grid = s.grid_view;
     const ScanParamsDF q = params_df(bp, s.pairsdf.p, s.df_lj_pairs, s.df_morse_pairs, s.esdf.p, s.griddf.p);
-    cuda_check(launch_grid_builddf(q, s.griddf.p, s.griddf64.p, &s.ctr.p->error_word, st), "grid build");
+    cuda_check(launch_grid_builddf(q, s.griddf.p, s.griddf64.p, &s.ctr.p->error_word,
+                                   s.far_used ? &s.far : nullptr, st), "grid build");
     s.griddf_built = true;
 }
 
