@@ -951,21 +951,22 @@ __device__ __forceinline__ void strip_masked(const ScanParamsDF& p, const unsign
         val[m] = NodeDF{sm.fx[m].value(), sm.fy[m].value(), sm.fz[m].value(), sm.ee[m].value()};
 }
 
-// The far sums at a block's Chebyshev points: blockIdx.y the block, a thread four
+// The far sums at a block's Chebyshev points: blockIdx.y the block, a thread NB
 // points along z.
+template <int NB>
 __global__ void __launch_bounds__(128) far_coef_kernel(const ScanParamsDF p, const FarViewDF f) {
     const FarBlock q = far_block(f, blockIdx.y);
-    const int t = blockIdx.x * 128 + threadIdx.x;   // < kFarP * kFarP * kFarP / 4
-    const int k0 = t % (kFarP / 4) * 4, j = t / (kFarP / 4) % kFarP, i = t / (kFarP / 4) / kFarP;
-    D z[4];
+    const int t = blockIdx.x * 128 + threadIdx.x;   // < kFarP * kFarP * kFarP / NB
+    const int k0 = t % (kFarP / NB) * NB, j = t / (kFarP / NB) % kFarP, i = t / (kFarP / NB) / kFarP;
+    D z[NB];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) z[m] = f.cheb[2][q.b[2] * kFarP + k0 + m];
-    NodeDF val[4];
-    strip_masked<4>(p, f.mask + (size_t)blockIdx.y * f.words, f.words, true,
+    for (int m = 0; m < NB; ++m) z[m] = f.cheb[2][q.b[2] * kFarP + k0 + m];
+    NodeDF val[NB];
+    strip_masked<NB>(p, f.mask + (size_t)blockIdx.y * f.words, f.words, true,
                                 f.cheb[0][q.b[0] * kFarP + i], f.cheb[1][q.b[1] * kFarP + j], z, val);
     NodeDF* o = f.coef + ((size_t)blockIdx.y * kFarP * kFarP + i * kFarP + j) * kFarP + k0;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) o[m] = val[m];
+    for (int m = 0; m < NB; ++m) o[m] = val[m];
 }
 
 // The near sums at a block's nodes, a thread four nodes along z.
@@ -1349,7 +1350,14 @@ bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float
 static cudaError_t launch_far(const ScanParamsDF& p, NodeDF* out, Node64* out64, const FarViewDF& f, cudaStream_t s) {
     const unsigned blocks = (unsigned)((long long)f.nb[0] * f.nb[1] * f.nb[2]);
     far_classify_kernel<<<blocks, 128, 0, s>>>(f, p.pairs, p.n_lj_pairs + p.n_morse_pairs);
-    far_coef_kernel<<<dim3(kFarP * kFarP * kFarP / 4 / 128, blocks), 128, 0, s>>>(p, f);
+    // Four points a thread share the x and y separations; grids of so few blocks
+    // that this would not fill the GPU once take one (slab of 16 px 10.7 -> 7.5
+    // ms, 24 px 13.3 -> 10.3 ms; 64 px 46.2 ms either way, 256 px 478 / 528 ms).
+    constexpr int kPoints = kFarP * kFarP * kFarP;
+    if (kPoints / 4 / 128 * (long long)blocks < 3ll * sm_count())
+        far_coef_kernel<1><<<dim3(kPoints / 128, blocks), 128, 0, s>>>(p, f);
+    else
+        far_coef_kernel<4><<<dim3(kPoints / 4 / 128, blocks), 128, 0, s>>>(p, f);
     far_near_kernel<<<dim3((unsigned)((f.max_strips + 127) / 128), blocks), 128, 0, s>>>(p, f, out);
     far_interp_kernel<<<dim3((unsigned)f.max_planes, blocks), 256, 0, s>>>(p, f, out, out64);
     return cudaGetLastError();
