@@ -22,6 +22,7 @@
 #include <cstring>
 #include <vector>
 
+#include "ieee64.cuh"
 #include "mafm_internal.h"
 
 struct mafm_flex {
@@ -104,40 +105,34 @@ __device__ __forceinline__ V3 sub3(V3 a, V3 b) { return V3{a.x - b.x, a.y - b.y,
 __device__ __forceinline__ V3 add3(V3 a, V3 b) { return V3{a.x + b.x, a.y + b.y, a.z + b.z}; }
 __device__ __forceinline__ V3 scal(double s, V3 a) { return V3{s * a.x, s * a.y, s * a.z}; }
 __device__ __forceinline__ V3 mul3(V3 a, double s) { return V3{a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ V3 div3(V3 a, double s) { return V3{a.x / s, a.y / s, a.z / s}; }
+__device__ __forceinline__ V3 div3(V3 a, double s) { return V3{div64(a.x, s), div64(a.y, s), div64(a.z, s)}; }
 __device__ __forceinline__ double dot3(V3 a, V3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ double len3(V3 a) { return sqrt(a.x * a.x + a.y * a.y + a.z * a.z); }
+__device__ __forceinline__ double len3(V3 a) { return sqrt64(a.x * a.x + a.y * a.y + a.z * a.z); }
 __device__ __forceinline__ V3 cross3(V3 a, V3 b) {
     return V3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
-__device__ __forceinline__ V3 normalized3(V3 a) {
-    const double l = len3(a);
-    if (l > 1e-10) return V3{a.x / l, a.y / l, a.z / l};
-    return V3{0, 0, 0};
-}
-
 // LJ (interactions.cpp:15-27) / Morse (:29-40): force on atom 1 of r_vec = x1 - x2.
 __device__ __forceinline__ V3 vdw_force(int kind, const double p[3], V3 r, double& e) {
     if (kind == MAFM_PAIR_LJ) {
         const double r_sqr = r.x * r.x + r.y * r.y + r.z * r.z;
         const double r6 = r_sqr * r_sqr * r_sqr;
-        const double ta = p[1] / (r6 * r6);
-        const double tb = p[0] / r6;
+        const double ta = div64(p[1], r6 * r6);
+        const double tb = div64(p[0], r6);
         e = ta - tb;
-        return scal((12 * ta - 6 * tb) / r_sqr, r);
+        return scal(div64(12 * ta - 6 * tb, r_sqr), r);
     }
     const double rl = len3(r);
     const double d = exp(-p[1] * (rl - p[2]));
     e = p[0] * (d * d - 2 * d + 1);
     const double f_abs = 2 * p[0] * p[1] * (d * d - d);
-    return scal(f_abs / rl, r);
+    return scal(div64(f_abs, rl), r);
 }
 
 // Coulomb (interactions.cpp:42-51).
 __device__ __forceinline__ V3 coul_force(double qq, V3 r, double& e) {
     const double rl = len3(r);
-    e = qq / rl;
-    return scal(qq / (rl * rl * rl), r);
+    e = div64(qq, rl);
+    return scal(div64(qq, rl * rl * rl), r);
 }
 
 struct FlexKernelArgs {
@@ -205,12 +200,12 @@ __device__ void eval_task(const FlexKernelArgs& A, const double* pe, int kind, i
         }
         case FT_TD_HARM: {  // TipHarmonicInteraction (interactions.cpp:252-266)
             const V3 r_vec = sub3(P3(0), P3(1));
-            const double r = sqrt(r_vec.x * r_vec.x + r_vec.y * r_vec.y);
+            const double r = sqrt64(r_vec.x * r_vec.x + r_vec.y * r_vec.y);
             const double dr = r - A.P.harm_r0;
             en[slot] = A.P.harm_k * dr * dr;
             V3 f{0, 0, 0};
             if (r > 1e-10) {
-                const double c = -2 * A.P.harm_k * dr / r;
+                const double c = div64(-2 * A.P.harm_k * dr, r);
                 f = V3{c * r_vec.x, c * r_vec.y, 0};
             }
             put3(res, slot, f);
@@ -222,7 +217,7 @@ __device__ void eval_task(const FlexKernelArgs& A, const double* pe, int kind, i
             const V3 r_vec = sub3(P3(i), P3(j));
             const double r = len3(r_vec);
             const double dr = r - r0;
-            put3(res, slot, scal(-2 * k * dr / r, r_vec));
+            put3(res, slot, scal(div64(-2 * k * dr, r), r_vec));
             break;
         }
         case FT_ANGLE: {    // HarmonicAngleInteraction (interactions.cpp:311-338)
@@ -231,15 +226,15 @@ __device__ void eval_task(const FlexKernelArgs& A, const double* pe, int kind, i
             const V3 r1_vec = sub3(P3(i1), P3(sh));
             const V3 r2_vec = sub3(P3(i2), P3(sh));
             const double r1 = len3(r1_vec), r2 = len3(r2_vec);
-            double cos_t = dot3(r1_vec, r2_vec) / (r1 * r2);
+            double cos_t = div64(dot3(r1_vec, r2_vec), r1 * r2);
             if (cos_t > 1) cos_t = 1;
             else if (cos_t < -1) cos_t = -1;
             const double theta = acos(cos_t);
             const double sin_t = sin(theta);
             const double d_theta = theta - theta0;
-            const double f_mul = -2 * k * d_theta / sin_t;
-            const V3 f1 = scal(-f_mul / r1, sub3(div3(r2_vec, r2), div3(mul3(r1_vec, cos_t), r1)));
-            const V3 f2 = scal(-f_mul / r2, sub3(div3(r1_vec, r1), div3(mul3(r2_vec, cos_t), r2)));
+            const double f_mul = div64(-2 * k * d_theta, sin_t);
+            const V3 f1 = scal(div64(-f_mul, r1), sub3(div3(r2_vec, r2), div3(mul3(r1_vec, cos_t), r1)));
+            const V3 f2 = scal(div64(-f_mul, r2), sub3(div3(r1_vec, r1), div3(mul3(r2_vec, cos_t), r2)));
             put3(res, slot, f1);
             put3(res, slot + 1, f2);
             put3(res, slot + 2, add3(f1, f2));
@@ -255,16 +250,16 @@ __device__ void eval_task(const FlexKernelArgs& A, const double* pe, int kind, i
             const V3 m_vec = cross3(r12, r23v);
             const V3 n_vec = cross3(r43, r23v);
             const double m = len3(m_vec), n = len3(n_vec);
-            const double tan_s = dot3(n_vec, r12) * r23 / dot3(m_vec, n_vec);
+            const double tan_s = div64(dot3(n_vec, r12) * r23, dot3(m_vec, n_vec));
             const double sigma = atan(tan_s);
             const double d_sigma = sigma - sigma0;
             const double f_mul = 2 * k * d_sigma;
-            put3(res, slot, scal(-f_mul * r23 / (m * m), m_vec));
-            put3(res, slot + 1, scal(-f_mul, sub3(scal(dot3(r43, r23v) / (n * n * r23), n_vec),
-                                                  scal(((r23 * r23) + dot3(r12, r23v)) / (m * m * r23), m_vec))));
-            put3(res, slot + 2, scal(-f_mul, add3(scal(dot3(r12, r23v) / (m * m * r23), m_vec),
-                                                  scal(((r23 * r23) - dot3(r43, r23v)) / (n * n * r23), n_vec))));
-            put3(res, slot + 3, scal(f_mul * r23 / (n * n), n_vec));
+            put3(res, slot, scal(div64(-f_mul * r23, m * m), m_vec));
+            put3(res, slot + 1, scal(-f_mul, sub3(scal(div64(dot3(r43, r23v), n * n * r23), n_vec),
+                                                  scal(div64((r23 * r23) + dot3(r12, r23v), m * m * r23), m_vec))));
+            put3(res, slot + 2, scal(-f_mul, add3(scal(div64(dot3(r12, r23v), m * m * r23), m_vec),
+                                                  scal(div64((r23 * r23) - dot3(r43, r23v), n * n * r23), n_vec))));
+            put3(res, slot + 3, scal(div64(f_mul * r23, n * n), n_vec));
             break;
         }
         case FT_PAIR_VDW: {
@@ -279,12 +274,12 @@ __device__ void eval_task(const FlexKernelArgs& A, const double* pe, int kind, i
         }
         case FT_SUBSTRATE: { // SubstrateInteraction (interactions.cpp:280-296); idx: the atom
             const double dz = pe[3 * idx + 2] - A.sub[3];
-            const double sig_z = A.sub[5] / dz;
+            const double sig_z = div64(A.sub[5], dz);
             const double sig_z2 = sig_z * sig_z;
             const double sig_z4 = sig_z2 * sig_z2;
             const double sig_z10 = sig_z4 * sig_z4 * sig_z2;
             double fterm = 0.0;
-            if (dz <= A.sub[4]) fterm += 4 * A.sub[0] / dz * (sig_z10 - sig_z4) + 2 * A.sub[1] * dz;
+            if (dz <= A.sub[4]) fterm += div64(4 * A.sub[0], dz) * (sig_z10 - sig_z4) + 2 * A.sub[1] * dz;
             // -0: adding it leaves x and y as they are, signed zeros too
             put3(res, slot, V3{-0.0, -0.0, fterm});
             break;
@@ -293,7 +288,7 @@ __device__ void eval_task(const FlexKernelArgs& A, const double* pe, int kind, i
             const int a = (int)dv.xy[3 * idx];
             const double rx = pe[3 * a] - dv.xy[3 * idx + 1];
             const double ry = pe[3 * a + 1] - dv.xy[3 * idx + 2];
-            const double r = sqrt(rx * rx + ry * ry);
+            const double r = sqrt64(rx * rx + ry * ry);
             const double c = -2 * A.sub_k;
             put3(res, slot, r > 1e-10 ? V3{c * rx, c * ry, 0.0} : V3{0.0, 0.0, 0.0});
             break;
@@ -332,10 +327,10 @@ struct FlexCtl {
 // memory; then one thread per atom and component adds the atom's slots in the
 // reference's order.  The minimiser's per-atom parts run one thread per
 // component, beside the convergence test on one warp and the power P on
-// another.  A flexible C10H8 + H2 (25 columns x 6 heights): 505 -> 19.3 ms;
+// another.  A flexible C10H8 + H2 (25 columns x 6 heights): 505 -> 18.5 ms;
 // before, a warp held a column, each lane evaluated its atoms' interactions
 // one after another (the tip's 43 on one lane), and the kinds diverged.
-__global__ void __launch_bounds__(32 * kFlexWarps) flex_kernel(const __grid_constant__ FlexKernelArgs A) {
+__global__ void __launch_bounds__(32 * kFlexWarps, 2) flex_kernel(const __grid_constant__ FlexKernelArgs A) {
     extern __shared__ __align__(16) double flex_smem[];
     __shared__ FlexCtl ctl;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -569,7 +564,7 @@ __global__ void __launch_bounds__(32 * kFlexWarps) flex_kernel(const __grid_cons
                                 continue;
                             }
                             const double lf = len3(v3(S.fsum + 3 * a));
-                            const double fh = lf > 1e-10 ? S.fsum[q] / lf : 0.0;
+                            const double fh = lf > 1e-10 ? div64(S.fsum[q], lf) : 0.0;
                             S.pe[q] = (1 - alpha) * S.vel[q] + (alpha * fh) * len3(v3(S.vel + 3 * a));
                         }
                     }

@@ -43,7 +43,7 @@ __device__ double interp64_quad(const GridView& g, double pos, int c, int quad, 
     const double q = pos - g.origin[a];
     double pb;
     if (g.orthogonal) {
-        pb = q / g.basis[4 * a];
+        pb = quo64(q, g.basis[4 * a]);
     } else {
         const double qx = __shfl_sync(0xffffffffu, q, quad), qy = __shfl_sync(0xffffffffu, q, quad + 1),
                      qz = __shfl_sync(0xffffffffu, q, quad + 2);
@@ -98,13 +98,13 @@ __device__ __forceinline__ AtomRec64 term64(const ScanParams& p, int j, int n, V
 // The XY spring (add_tip_dummy): what is added to component c.
 __device__ __forceinline__ double spring64(const ScanParams& p, V3 tip, V3 dum, int c) {
     const double rx = dum.x - tip.x, ry = dum.y - tip.y;
-    const double rr = sqrt(rx * rx + ry * ry);
+    const double rr = root64(rx * rx + ry * ry);
     const double dr = rr - p.harm_r0;
     double add = -0.0;                      // no z force
     if (c == 3) {
         add = p.harm_k * dr * dr;
     } else if (c < 2 && rr > 1e-10) {
-        const double s = -2 * p.harm_k * dr / rr;
+        const double s = quo64(-2 * p.harm_k * dr, rr);
         add = -(s * (c == 0 ? rx : ry));
     }
     return add;
@@ -129,9 +129,9 @@ __device__ __forceinline__ double spring64(const ScanParams& p, V3 tip, V3 dum, 
 // the minimiser and the sums; all four compute the terms, van der Waals and
 // Coulomb records on different warps, the last one the spring.
 //
-// 51 x 51 x 11 graphene (2,601 columns, G = 8): 178 -> 30.5 ms; one thread per
+// 51 x 51 x 11 graphene (2,601 columns, G = 8): 178 -> 26 ms; one thread per
 // column used 21 of the 152 SMs there, and kept half of its lanes waiting.  301
-// columns of the 60-atom cluster x 41 (W = 4): 255 -> 152 ms; one warp per
+// columns of the 60-atom cluster x 41 (W = 4): 255 -> 131 ms; one warp per
 // column took 219 ms.
 template <int G, int W>
 __global__ void __launch_bounds__(32 * W) relax64_kernel(const __grid_constant__ ScanParams p, mafm_point* out,
@@ -396,16 +396,16 @@ __global__ void __launch_bounds__(32 * W) relax64_kernel(const __grid_constant__
                 fs = fs + F;
                 es = es + E;
                 vs = vs + u;
-                const double s6 = dt / 6.0;
+                const double s6 = quo64(dt, 6.0);
                 pp = pp + s6 * vs;
                 v = v + s6 * fs;
-                SF = fs / 6.0;
-                SE = es / 6.0;
+                SF = quo64(fs, 6.0);
+                SE = quo64(es, 6.0);
             }
         }
         // FIREMinimisation / SDMinimisation (minimiser.cpp:39-129)
         if (c == 3) SF = 0;                 // the energy's lane has no vector component
-        const double fl = sqrt(dot(SF, SF));
+        const double fl = root64(dot(SF, SF));
         const double ediff = SE - energy;
         if (act) energy = SE;
         bool conv;
@@ -417,8 +417,8 @@ __global__ void __launch_bounds__(32 * W) relax64_kernel(const __grid_constant__
             if (go) pp = pp + p.dt * SF;
         } else {
             const double pw = dot(v, SF);
-            const double vl = sqrt(dot(v, v));
-            const double fh = fl > 1e-10 ? SF / fl : 0.0;
+            const double vl = root64(dot(v, v));
+            const double fh = fl > 1e-10 ? quo64(SF, fl) : 0.0;
             const double mixed = (1.0 - alpha) * v + alpha * fh * vl;
             if (go) {
                 if (pw < 0.0) {
@@ -577,7 +577,7 @@ static cudaError_t launch_relax64_g(const ScanParams& p, mafm_point* out, RunCou
 // FP64 instruction every 19 cycles and a warp one every 64).  Four lanes cost
 // no more FP64 instructions per column than one, 8 / 16 / 32 lanes 9 / 38 / 95 %
 // more (72 LJ terms), because the in-order sums leave more of them idle.
-// Measured, G = 4 / 8 / 16 / 32: 2,601 columns (graphene, 11 heights) 42.1 /
+// Measured with the divide and square root operators, G = 4 / 8 / 16 / 32: 2,601 columns (graphene, 11 heights) 42.1 /
 // 30.5 / 33.9 / 48.0 ms; 90,000 (cluster, 2 heights) 523 / 647 / 784 / 1071 ms.
 // Four warps per column while there are few columns (and terms to share):
 // cluster, 41 heights, one warp / four warps: 1 column 126 / 78 ms, 301 218 /

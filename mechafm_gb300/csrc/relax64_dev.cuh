@@ -12,6 +12,7 @@
 //   trilinear grid lookup      force_grid.cpp:88-275
 #pragma once
 
+#include "ieee64.cuh"
 #include "mafm_internal.h"
 #include "relax_tpl.cuh"
 
@@ -20,32 +21,44 @@ namespace {
 
 using V3 = V3T<double>;
 
+// Quotient and root of the FP64 kernels (the same bits either way).  The double-
+// float kernel's own re-relaxation of a few columns keeps the operators: div64
+// would raise the registers of the whole kernel.
+#ifdef MAFM_PLAIN_DIV64
+__device__ __forceinline__ double quo64(double a, double b) { return a / b; }
+__device__ __forceinline__ double root64(double x) { return sqrt(x); }
+#else
+__device__ __forceinline__ double quo64(double a, double b) { return div64(a, b); }
+__device__ __forceinline__ double root64(double x) { return sqrt64(x); }
+#endif
+__device__ __forceinline__ double length64(V3 v) { return root64(v.x * v.x + v.y * v.y + v.z * v.z); }
+
 // LJInteraction::eval / MorseInteraction::eval; r = tip - (atom + shift).
 __device__ __forceinline__ void vdw64(int kind, double p0, double p1, double p2, V3 r, V3& f,
                                       double& e) {
     if (kind == MAFM_PAIR_LJ) {
         double r_sqr = r.x * r.x + r.y * r.y + r.z * r.z;
         double r6 = r_sqr * r_sqr * r_sqr;
-        double term_a = p1 / (r6 * r6);
-        double term_b = p0 / r6;
+        double term_a = quo64(p1, r6 * r6);
+        double term_b = quo64(p0, r6);
         e = term_a - term_b;
-        double s = (12 * term_a - 6 * term_b) / r_sqr;
+        double s = quo64(12 * term_a - 6 * term_b, r_sqr);
         f.x = s * r.x; f.y = s * r.y; f.z = s * r.z;
     } else {
-        double rl = len3(r);
+        double rl = length64(r);
         double d = exp(-p1 * (rl - p2));
         e = p0 * (d * d - 2 * d + 1);
         double f_abs = 2 * p0 * p1 * (d * d - d);
-        double s = f_abs / rl;
+        double s = quo64(f_abs, rl);
         f.x = s * r.x; f.y = s * r.y; f.z = s * r.z;
     }
 }
 
 // CoulombInteraction::eval
 __device__ __forceinline__ void coul64(double qq, V3 r, V3& f, double& e) {
-    double rl = len3(r);
-    e = qq / rl;
-    double s = qq / (rl * rl * rl);
+    double rl = length64(r);
+    e = quo64(qq, rl);
+    double s = quo64(qq, rl * rl * rl);
     f.x = s * r.x; f.y = s * r.y; f.z = s * r.z;
 }
 
@@ -76,7 +89,7 @@ __device__ void interp64(const GridView& g, V3 pos, V3& f, double& e, int& outsi
     V3 q = {pos.x - g.origin[0], pos.y - g.origin[1], pos.z - g.origin[2]};
     V3 pb;
     if (g.orthogonal) {
-        pb.x = q.x / g.basis[0]; pb.y = q.y / g.basis[4]; pb.z = q.z / g.basis[8];
+        pb.x = quo64(q.x, g.basis[0]); pb.y = quo64(q.y, g.basis[4]); pb.z = quo64(q.z, g.basis[8]);
     } else {
         pb.x = g.inv[0] * q.x + g.inv[1] * q.y + g.inv[2] * q.z;
         pb.y = g.inv[3] * q.x + g.inv[4] * q.y + g.inv[5] * q.z;
@@ -124,12 +137,12 @@ __device__ __forceinline__ void add_tip_dummy(const ScanParams& p, V3 tip, V3 du
         F.x -= f.x; F.y -= f.y; F.z -= f.z; E += e;
     }
     double rx = dum.x - tip.x, ry = dum.y - tip.y;
-    double rr = sqrt(rx * rx + ry * ry);
+    double rr = root64(rx * rx + ry * ry);
     double dr = rr - p.harm_r0;
     double eh = p.harm_k * dr * dr;
     double fx = 0, fy = 0;
     if (rr > 1e-10) {
-        double s = -2 * p.harm_k * dr / rr;
+        double s = quo64(-2 * p.harm_k * dr, rr);
         fx = s * rx; fy = s * ry;
     }
     F.x -= fx; F.y -= fy; F.z -= 0.0;

@@ -37,6 +37,7 @@
 #include <cmath>
 #include <cstdlib>
 
+#define MAFM_PLAIN_DIV64   // see relax64_dev.cuh
 #include "mafm_df.h"
 #include "relax64_dev.cuh"
 #include "relax_tpl.cuh"
