@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 
 #define MAFM_PLAIN_DIV64   // see relax64_dev.cuh
 #include "mafm_df.h"
@@ -48,15 +49,12 @@ namespace {
 using D = dfloat;
 using V3D = V3T<dfloat>;
 
-// One tip–atom term for the separation d = tip - atom: LJ (interactions.cpp:
-// 15-27) or Morse (:29-40), plus Coulomb (:42-51) when coul.  1/r comes from
-// a double-float rsqrt; f is the force on the tip.
-__device__ __forceinline__ void pair_df(int kind, D p0, D p1, D p2, bool coul, D qq, V3D d,
-                                        V3D& f, D& e) {
-    const D r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+// One term at the distance squared r2: LJ (interactions.cpp:15-27) or Morse
+// (:29-40), plus Coulomb (:42-51) when coul.  1/r comes from a double-float rsqrt;
+// the force on the first particle is s times the separation.
+__device__ __forceinline__ void pair_df(int kind, D p0, D p1, D p2, bool coul, D qq, D r2, D& s, D& e) {
     const D ir = dfl_rsqrt(r2);
     const D ir2 = ir * ir;
-    D s;
     if (kind == MAFM_PAIR_LJ) {
         const D ir6 = ir2 * ir2 * ir2;
         const D a = p1 * (ir6 * ir6);   // es12 / r^12
@@ -75,9 +73,6 @@ __device__ __forceinline__ void pair_df(int kind, D p0, D p1, D p2, bool coul, D
         e = e + ec;
         s = s + ec * ir2;
     }
-    f.x = s * d.x;
-    f.y = s * d.y;
-    f.z = s * d.z;
 }
 
 using D2 = dfloat2;
@@ -325,16 +320,82 @@ __device__ void interp_df_grid(const GridViewDF& g, V3D pos, V3D& f, D& e, int& 
     e = out[3];
 }
 
+// Vectors of a column's state.  With G >= 4 lanes per column lane c of every quad
+// holds component c (x, y, z; lane 3 goes along with z, and holds E where forces
+// are summed), so that the vector arithmetic of the minimiser, which every lane of
+// the group would otherwise repeat, costs a third; with fewer lanes every lane
+// holds all three.  The operations of a component are the same: the same bits.
+// 101 x 101 graphene (G = 4) 107.3 -> 104.7 ms, 40 x 40 (G = 8) 11.8 -> 10.8 ms.
+struct QuadDF {
+    D c;
+};
+template <int G>
+using VecDF = std::conditional_t<(G >= 4), QuadDF, V3D>;
+
+// Component m of a quad, on all of its lanes.
+__device__ __forceinline__ D quad_get(D v, int m, unsigned gmask) {
+    const int src = ((int)threadIdx.x & 28) | m;
+    return D(__shfl_sync(gmask, v.h, src), __shfl_sync(gmask, v.l, src));
+}
+template <int G>
+__device__ __forceinline__ V3D whole(VecDF<G> v, unsigned gmask) {
+    if constexpr (G >= 4) return {quad_get(v.c, 0, gmask), quad_get(v.c, 1, gmask), quad_get(v.c, 2, gmask)};
+    else return v;
+}
+template <int G>
+__device__ __forceinline__ VecDF<G> own(V3D v) {
+    if constexpr (G >= 4) {
+        const int c = threadIdx.x & 3;
+        return {c == 0 ? v.x : c == 1 ? v.y : v.z};
+    } else {
+        return v;
+    }
+}
+// f of the components of a, b
+template <class F>
+__device__ __forceinline__ QuadDF vmap(QuadDF a, QuadDF b, F f) { return {f(a.c, b.c)}; }
+template <class F>
+__device__ __forceinline__ V3D vmap(V3D a, V3D b, F f) { return {f(a.x, b.x), f(a.y, b.y), f(a.z, b.z)}; }
+// a . b, the products added in the order x, y, z
+template <int G>
+__device__ __forceinline__ D vdot(VecDF<G> a, VecDF<G> b, unsigned gmask) {
+    if constexpr (G >= 4) {
+        const D s = a.c * b.c;
+        return quad_get(s, 0, gmask) + quad_get(s, 1, gmask) + quad_get(s, 2, gmask);
+    } else {
+        return a.x * b.x + a.y * b.y + a.z * b.z;
+    }
+}
+
+// The sums over the G >= 4 lanes of a group of fx, fy, fz and e, one on each lane
+// of a quad, each added as group_sum adds it.
+template <int G>
+__device__ __forceinline__ D quad_sum(D fx, D fy, D fz, D e, int sub, unsigned gmask) {
+    auto other = [&](D v, int m) {
+        return D(__shfl_xor_sync(gmask, v.h, m), __shfl_xor_sync(gmask, v.l, m));
+    };
+    const bool odd = sub & 1, up = sub & 2;
+    const D a = (odd ? fy : fx) + other(odd ? fx : fy, 1);
+    const D b = (odd ? e : fz) + other(odd ? fz : e, 1);
+    D v = (up ? b : a) + other(up ? a : b, 2);
+#pragma unroll
+    for (int m = 4; m < G; m <<= 1) v = v + other(v, m);
+    return v;
+}
+
 // System::evalTipSurfaceForces (system.cpp:41-51): the tip–surface force and
 // energy at tip, by the G lanes of a group (lane sub of the group takes the
 // term pairs sub, sub + G, ...; the external field on lane 0).  The loop over
 // terms is the same for every group of a scan.
 template <int G>
-__device__ __forceinline__ void ts_df(const ScanParamsDF& p, V3D tip, int sub, unsigned gmask,
-                                      V3D& F, D& E, int& outside, unsigned& err) {
+__device__ __forceinline__ void ts_df(const ScanParamsDF& p, VecDF<G> at, int sub, unsigned gmask,
+                                      VecDF<G>& F, D& E, int& outside, unsigned& err) {
+    const V3D tip = whole<G>(at, gmask);
     if (p.ts_mode == 2) {
         // the rigid grid alone; every lane of the group looks it up
-        interp_df_grid(p.grid, tip, F, E, outside, err);
+        V3D f;
+        interp_df_grid(p.grid, tip, f, E, outside, err);
+        F = own<G>(f);
         return;
     }
     LazySum2 fx, fy, fz, ee;
@@ -353,28 +414,50 @@ __device__ __forceinline__ void ts_df(const ScanParamsDF& p, V3D tip, int sub, u
         fz.add(D2{make_float2(f.z.h, 0.0f), make_float2(f.z.l, 0.0f)});
         ee.add(D2{make_float2(e.h, 0.0f), make_float2(e.l, 0.0f)});
     }
-    F = {group_sum<G>(fx.value(), sub, gmask), group_sum<G>(fy.value(), sub, gmask),
-         group_sum<G>(fz.value(), sub, gmask)};
-    E = group_sum<G>(ee.value(), sub, gmask);
+    if constexpr (G >= 4) {
+        const D v = quad_sum<G>(fx.value(), fy.value(), fz.value(), ee.value(), sub, gmask);
+        F = {v};
+        E = quad_get(v, 3, gmask);
+    } else {
+        F = {group_sum<G>(fx.value(), sub, gmask), group_sum<G>(fy.value(), sub, gmask),
+             group_sum<G>(fz.value(), sub, gmask)};
+        E = group_sum<G>(ee.value(), sub, gmask);
+    }
 }
 
 // The tip–dummy terms and the XY spring, added in Eval64::all's order
 // (simulation.cpp:503-515, interactions.cpp:252-266).
-__device__ __forceinline__ void tip_dummy_df(const ScanParamsDF& p, V3D tip, V3D dum, V3D& F,
-                                             D& E) {
-    const V3D r = {dum.x - tip.x, dum.y - tip.y, dum.z - tip.z};
-    V3D f;
-    D e;
-    pair_df(p.td_kind, p.td_p[0], p.td_p[1], p.td_p[2], p.td_coul != 0, p.td_qq, r, f, e);
-    F.x = F.x - f.x; F.y = F.y - f.y; F.z = F.z - f.z;
+template <int G>
+__device__ __forceinline__ void tip_dummy_df(const ScanParamsDF& p, VecDF<G> tip, VecDF<G> dum, unsigned gmask,
+                                             VecDF<G>& F, D& E) {
+    const VecDF<G> r = vmap(dum, tip, [](D d, D x) { return d - x; });
+    D xx, yy, r2;
+    if constexpr (G >= 4) {
+        const D q = r.c * r.c;
+        xx = quad_get(q, 0, gmask);
+        yy = quad_get(q, 1, gmask);
+        r2 = xx + yy + quad_get(q, 2, gmask);
+    } else {
+        xx = r.x * r.x;
+        yy = r.y * r.y;
+        r2 = xx + yy + r.z * r.z;
+    }
+    D s, e;
+    pair_df(p.td_kind, p.td_p[0], p.td_p[1], p.td_p[2], p.td_coul != 0, p.td_qq, r2, s, e);
+    F = vmap(F, r, [&](D f, D x) { return f - s * x; });
     E = E + e;
-    const D rr = dfl_sqrt(r.x * r.x + r.y * r.y);
+    const D rr = dfl_sqrt(xx + yy);
     const D dr = rr - p.harm_r0;
     E = E + p.harm_k * dr * dr;
     if (rr > D(1e-10)) {
-        const D s = -(p.harm_k * 2.0f) * dr / rr;
-        F.x = F.x - s * r.x;
-        F.y = F.y - s * r.y;
+        const D h = -(p.harm_k * 2.0f) * dr / rr;
+        if constexpr (G >= 4) {
+            const D f = F.c - h * r.c;
+            if ((threadIdx.x & 3) < 2) F.c = f;
+        } else {
+            F.x = F.x - h * r.x;
+            F.y = F.y - h * r.y;
+        }
     }
 }
 
@@ -382,9 +465,10 @@ enum : int { DF_EVAL0 = 0, DF_EVAL1 = 1, DF_EVAL2 = 2, DF_EVAL3 = 3, DF_OUT = 4 
 
 // One lane's column: the state fire_t / sd_t keep in locals, held across
 // slots.  u is the midpoint v2 / the RK4 v_k; vs, fs, es the RK4 sums.
+template <int G>
 struct LaneDF {
     int col, scan, k, n, nnn, phase, tie, outside;
-    V3D tip, vel, dum, ex, u, vs, fs;
+    VecDF<G> tip, vel, dum, ex, u, vs, fs;
     D energy, es, alpha, dt;
 };
 
@@ -468,7 +552,7 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
     const unsigned long long t0 = df_global_ns();
     unsigned ticks = 0;
 
-    LaneDF s;
+    LaneDF<G> s;
     s.col = -1;
     s.scan = 0;
     s.tie = 0;
@@ -532,9 +616,9 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
                     const int i = s.col / P.ny, j = s.col % P.ny;
                     D x, y;
                     dummy_xy_t(P, wrap, D(i) * P.dx, D(j) * P.dy, x, y);
-                    s.dum = {x, y, P.zhigh};
-                    s.tip = {x, y, P.zhigh - P.tip_dummy_d};
-                    s.vel = {D(0), D(0), D(0)};
+                    s.dum = own<G>(V3D{x, y, P.zhigh});
+                    s.tip = own<G>(V3D{x, y, P.zhigh - P.tip_dummy_d});
+                    s.vel = own<G>(V3D{D(0), D(0), D(0)});
                     s.energy = D(0);
                     s.k = 0;
                     s.tie = 0;
@@ -559,7 +643,7 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
         if ((s.phase == DF_EVAL0 || s.phase == DF_OUT) && (ticks & P.stage_mask)) continue;
 
         // ---- one evaluation per lane ----
-        V3D F;
+        VecDF<G> F;
         D E;
         ts_df<G>(P, s.ex, sub, gmask, F, E, s.outside, err);
         if (sub == 0) {
@@ -570,11 +654,12 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
             // System::getOutput (system.cpp:28-51)
             int st = (s.n >= P.maxsteps ? MAFM_PT_MAXSTEPS : 0) | (s.tie ? MAFM_PT_NEAR_TIE : 0) |
                      (s.outside ? MAFM_PT_OUTSIDE : 0);
-            if (!dfl_isfinite(F.x) || !dfl_isfinite(F.y) || !dfl_isfinite(F.z) || !dfl_isfinite(E))
+            const V3D f = whole<G>(F, gmask), tip = whole<G>(s.tip, gmask);
+            if (!dfl_isfinite(f.x) || !dfl_isfinite(f.y) || !dfl_isfinite(f.z) || !dfl_isfinite(E))
                 st |= MAFM_PT_NONFINITE;
             mafm_point r;
-            r.tip[0] = to_double(s.tip.x); r.tip[1] = to_double(s.tip.y); r.tip[2] = to_double(s.tip.z);
-            r.force[0] = to_double(F.x); r.force[1] = to_double(F.y); r.force[2] = to_double(F.z);
+            r.tip[0] = to_double(tip.x); r.tip[1] = to_double(tip.y); r.tip[2] = to_double(tip.z);
+            r.force[0] = to_double(f.x); r.force[1] = to_double(f.y); r.force[2] = to_double(f.z);
             r.energy = to_double(E);
             r.steps = s.n;
             r.status = st;
@@ -584,8 +669,15 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
                 status_or |= (unsigned)st;
             }
             // System::lowerTip (system.hpp:51-54)
-            s.dum.z = s.dum.z - P.dz;
-            s.tip.z = s.tip.z - P.dz;
+            if constexpr (G >= 4) {
+                if ((lane & 3) >= 2) {
+                    s.dum.c = s.dum.c - P.dz;
+                    s.tip.c = s.tip.c - P.dz;
+                }
+            } else {
+                s.dum.z = s.dum.z - P.dz;
+                s.tip.z = s.tip.z - P.dz;
+            }
             if (++s.k < P.nz) {
                 start_level();
             } else {
@@ -593,59 +685,58 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
             }
             continue;
         }
-        tip_dummy_df(P, s.ex, s.dum, F, E);
+        tip_dummy_df<G>(P, s.ex, s.dum, gmask, F, E);
 
         // ---- the integrator stage this evaluation belongs to (integrators.cpp:8-111) ----
         bool step_done = false;
-        V3D SF = F;
+        VecDF<G> SF = F;
         D SE = E;
         const D dt = s.dt;
+        // x + w y of every component
+        auto step = [](VecDF<G> x, D w, VecDF<G> y) { return vmap(x, y, [&](D a, D b) { return a + w * b; }); };
         if (P.minimiser == MAFM_MIN_SD) {
             step_done = true;
         } else if (P.integrator == MAFM_INT_EULER) {
-            const V3D pp = s.tip, v = s.vel;
-            s.tip = {pp.x + dt * v.x, pp.y + dt * v.y, pp.z + dt * v.z};
-            s.vel = {v.x + dt * F.x, v.y + dt * F.y, v.z + dt * F.z};
+            s.tip = step(s.tip, dt, s.vel);
+            s.vel = step(s.vel, dt, F);
             step_done = true;
         } else if (P.integrator == MAFM_INT_MIDPOINT) {
             const D h(__fmul_rn(dt.h, 0.5f), __fmul_rn(dt.l, 0.5f));   // dt / 2, exactly
             if (s.phase == DF_EVAL0) {
-                const V3D pp = s.tip, v = s.vel;
-                s.ex = {pp.x + h * v.x, pp.y + h * v.y, pp.z + h * v.z};
-                s.u = {v.x + h * F.x, v.y + h * F.y, v.z + h * F.z};
+                s.ex = step(s.tip, h, s.vel);
+                s.u = step(s.vel, h, F);
                 s.phase = DF_EVAL1;
             } else {
-                const V3D pp = s.tip, v = s.vel;
-                s.tip = {pp.x + dt * s.u.x, pp.y + dt * s.u.y, pp.z + dt * s.u.z};
-                s.vel = {v.x + dt * F.x, v.y + dt * F.y, v.z + dt * F.z};
+                s.tip = step(s.tip, dt, s.u);
+                s.vel = step(s.vel, dt, F);
                 step_done = true;
             }
         } else {   // RK4
             const D h(__fmul_rn(dt.h, 0.5f), __fmul_rn(dt.l, 0.5f));   // dt / 2, exactly
-            const V3D pp = s.tip, v = s.vel;
+            auto sum = [](VecDF<G> x, VecDF<G> y) { return vmap(x, y, [](D a, D b) { return a + b; }); };
             if (s.phase == DF_EVAL0) {
-                s.fs = F; s.es = E; s.vs = v;
-                s.ex = {pp.x + h * v.x, pp.y + h * v.y, pp.z + h * v.z};
-                s.u = {v.x + h * F.x, v.y + h * F.y, v.z + h * F.z};
+                s.fs = F; s.es = E; s.vs = s.vel;
+                s.ex = step(s.tip, h, s.vel);
+                s.u = step(s.vel, h, F);
                 s.phase = DF_EVAL1;
             } else if (s.phase == DF_EVAL1 || s.phase == DF_EVAL2) {
                 const D two(2);
-                s.fs = {s.fs.x + two * F.x, s.fs.y + two * F.y, s.fs.z + two * F.z};
+                s.fs = step(s.fs, two, F);
                 s.es = s.es + two * E;
-                s.vs = {s.vs.x + two * s.u.x, s.vs.y + two * s.u.y, s.vs.z + two * s.u.z};
+                s.vs = step(s.vs, two, s.u);
                 const D w = s.phase == DF_EVAL1 ? h : dt;
-                s.ex = {pp.x + w * s.u.x, pp.y + w * s.u.y, pp.z + w * s.u.z};
-                s.u = {v.x + w * F.x, v.y + w * F.y, v.z + w * F.z};
+                s.ex = step(s.tip, w, s.u);
+                s.u = step(s.vel, w, F);
                 s.phase = s.phase + 1;
             } else {
-                s.fs = {s.fs.x + F.x, s.fs.y + F.y, s.fs.z + F.z};
+                s.fs = sum(s.fs, F);
                 s.es = s.es + E;
-                s.vs = {s.vs.x + s.u.x, s.vs.y + s.u.y, s.vs.z + s.u.z};
+                s.vs = sum(s.vs, s.u);
                 const D s6 = dt / D(6);
                 const D sixth = D(1.0 / 6.0);
-                s.tip = {pp.x + s6 * s.vs.x, pp.y + s6 * s.vs.y, pp.z + s6 * s.vs.z};
-                s.vel = {v.x + s6 * s.fs.x, v.y + s6 * s.fs.y, v.z + s6 * s.fs.z};
-                SF = {s.fs.x * sixth, s.fs.y * sixth, s.fs.z * sixth};
+                s.tip = step(s.tip, s6, s.vs);
+                s.vel = step(s.vel, s6, s.fs);
+                SF = vmap(s.fs, s.fs, [&](D a, D) { return a * sixth; });
                 SE = s.es * sixth;
                 step_done = true;
             }
@@ -657,7 +748,7 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
         const D prev = s.energy;
         s.energy = SE;
         const D ediff = SE - prev;
-        const D fl = len3(SF);
+        const D fl = dfl_sqrt(vdot<G>(SF, SF, gmask));
         bool conv;
         {
             // checkConvergence (minimiser.cpp:15-37), and its near-ties
@@ -681,26 +772,25 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
             continue;
         }
         if (P.minimiser == MAFM_MIN_SD) {
-            s.tip = {s.tip.x + P.dt * SF.x, s.tip.y + P.dt * SF.y, s.tip.z + P.dt * SF.z};
+            s.tip = vmap(s.tip, SF, [&](D x, D f) { return x + P.dt * f; });
         } else {
-            const V3D w = s.vel;
-            const D pw = w.x * SF.x + w.y * SF.y + w.z * SF.z;
-            V3D fh = {D(0), D(0), D(0)};
+            const VecDF<G> w = s.vel;
+            const D pw = vdot<G>(w, SF, gmask);
+            VecDF<G> fh = own<G>(V3D{D(0), D(0), D(0)});
             if (fl > D(1e-10)) {
                 const D ifl = dfl_rcp(fl);
-                fh = {SF.x * ifl, SF.y * ifl, SF.z * ifl};
+                fh = vmap(SF, SF, [&](D f, D) { return f * ifl; });
             }
-            const D vl = len3(w);
+            const D vl = dfl_sqrt(vdot<G>(w, w, gmask));
             s.tie |= dfl_fabs(pw) < vl * (P.tie.p_f + P.tie.p_v * fl);
             if (s.tie && repair_list) {
                 give_up();
                 continue;
             }
             const D one_a = D(1) - s.alpha;
-            s.vel = {one_a * w.x + s.alpha * fh.x * vl, one_a * w.y + s.alpha * fh.y * vl,
-                     one_a * w.z + s.alpha * fh.z * vl};
+            s.vel = vmap(w, fh, [&](D x, D f) { return one_a * x + s.alpha * f * vl; });
             if (pw < D(0)) {
-                s.vel = {D(0), D(0), D(0)};
+                s.vel = own<G>(V3D{D(0), D(0), D(0)});
                 s.nnn = 0;
                 s.dt = s.dt * D(0.5);
                 s.alpha = D(0.1);
