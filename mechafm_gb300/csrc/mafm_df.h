@@ -135,7 +135,8 @@ struct FarViewDF {
     unsigned* mask;                  // words per block
     NodeDF* coef;                    // kFarPoints^3 per block
 };
-bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float>& xyz, FarPlanDF& plan);
+bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float>& xyz, int n_lj,
+                 FarPlanDF& plan);
 
 // Simulation::buildTipGridInteractions (simulation.cpp:420-501) in
 // double-float: the rigid grid of geometry p.grid (p.ts_mode 0 or 1: the

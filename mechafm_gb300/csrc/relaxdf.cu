@@ -954,9 +954,12 @@ __global__ void nodes_df_to_64_kernel(const NodeDF* in, Node64* out, long long n
 // block's interval (scaled to [-1, 1]) on which the term has its nearest
 // singularity has a half axis of at least kFarAxis: a term (r^-1 to r^-14) is then
 // interpolated to 1e-15 of itself or better (the r^-14 part, which converges
-// slowest, is below 1e-4 of its r^-7 part there).  Blocks, Chebyshev points and
-// the interpolation weights are laid out once (plan_far_df); every build
-// classifies the records and evaluates all of it.
+// slowest, is below 1e-4 of its r^-7 part there).  Morse records are always near:
+// exp(-2 a r) over an interval of half length h converges with a h, whatever the
+// distance, and a term with a = 2 A^-1 over 3.2 A would be good to 1e-7 of itself
+// only, which counts where every term is weak.  Blocks, Chebyshev points and the
+// interpolation weights are laid out once (plan_far_df); every build classifies
+// the records and evaluates all of it.
 //
 // Slab of 9,216 records: 64 x 64 px (157 x 157 x 141 nodes) 270 -> 46 ms, 256 x 256
 // px (541 x 541 x 141) 3198 -> 479 ms; and fewer roundings per node: the relaxed
@@ -997,8 +1000,9 @@ __device__ __forceinline__ FarBlock far_block(const FarViewDF& f, int id) {
     return q;
 }
 
-// One bit per record and block: set when either of its terms is near.
-__global__ void far_classify_kernel(const FarViewDF f, const TermPairDF* pairs, int n_rec) {
+// One bit per record and block: set when the record is a Morse one (past the first
+// n_lj) or either of its terms is near.
+__global__ void far_classify_kernel(const FarViewDF f, const TermPairDF* pairs, int n_lj, int n_rec) {
     const FarBlock q = far_block(f, blockIdx.x);
     float c[3], h[3];
     for (int a = 0; a < 3; ++a) {
@@ -1010,7 +1014,7 @@ __global__ void far_classify_kernel(const FarViewDF f, const TermPairDF* pairs, 
         for (int k = 0; k < 32 && 32 * w + k < n_rec; ++k) {
             const TermPairDF& t = pairs[32 * w + k];
             const float a0[3] = {t.xh.x, t.yh.x, t.zh.x}, a1[3] = {t.xh.y, t.yh.y, t.zh.y};
-            if (near_box(a0, c, h) || near_box(a1, c, h)) bits |= 1u << k;
+            if (32 * w + k >= n_lj || near_box(a0, c, h) || near_box(a1, c, h)) bits |= 1u << k;
         }
         f.mask[(size_t)blockIdx.x * f.words + w] = bits;
     }
@@ -1318,7 +1322,8 @@ cudaError_t launch_nodes_to_df(const Node64* in, NodeDF* out, long long n, cudaS
 // least by the estimate below, none across a jump of the wrapped positions, and
 // for every axis Chebyshev points and the weights of the block's nodes.  xyz: the
 // positions of the records' two terms.
-bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float>& xyz, FarPlanDF& plan) {
+bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float>& xyz, int n_lj,
+                 FarPlanDF& plan) {
     const long long n_rec = (long long)xyz.size() / 6;
     if (n_rec < 64) return false;
     if (p.tip_pbc)
@@ -1384,7 +1389,7 @@ bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float
                 h[a] = (float)b.second;
             }
             for (long long r = 0; r < n_rec; r += step, ++tried)
-                near += near_box(&xyz[6 * r], c, h) || near_box(&xyz[6 * r + 3], c, h);
+                near += r >= n_lj || near_box(&xyz[6 * r], c, h) || near_box(&xyz[6 * r + 3], c, h);
         }
         near *= (double)n_rec / tried;
         // per node the interpolation costs about four records
@@ -1440,7 +1445,7 @@ bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float
 
 static cudaError_t launch_far(const ScanParamsDF& p, NodeDF* out, Node64* out64, const FarViewDF& f, cudaStream_t s) {
     const unsigned blocks = (unsigned)((long long)f.nb[0] * f.nb[1] * f.nb[2]);
-    far_classify_kernel<<<blocks, 128, 0, s>>>(f, p.pairs, p.n_lj_pairs + p.n_morse_pairs);
+    far_classify_kernel<<<blocks, 128, 0, s>>>(f, p.pairs, p.n_lj_pairs, p.n_lj_pairs + p.n_morse_pairs);
     // Four points a thread share the x and y separations; grids of so few blocks
     // that this would not fill the GPU once take one (slab of 16 px 10.7 -> 7.5
     // ms, 24 px 13.3 -> 10.3 ms; 64 px 46.2 ms either way, 256 px 478 / 528 ms).

@@ -609,7 +609,7 @@ void ensure_grid(mafm_scan& s, bool fp64, cudaStream_t st, bool rebuild = false)
 void ensure_far_plan(mafm_scan& s, cudaStream_t st) {
     if (s.far_planned) return;
     FarPlanDF plan;
-    if (plan_far_df(build_grid_params(s), s.grid_view, s.df_xyz, plan)) {
+    if (plan_far_df(build_grid_params(s), s.grid_view, s.df_xyz, s.df_lj_pairs, plan)) {
         std::vector<unsigned char> host;
         auto piece = [&](const void* p, size_t bytes) {
             const size_t at = (host.size() + 63) & ~(size_t)63;
@@ -633,9 +633,18 @@ void ensure_far_plan(mafm_scan& s, cudaStream_t st) {
             if (a == 0) s.far.max_planes = most;
             strips *= a == 2 ? (most + 3) / 4 : most;
         }
-        s.far_tables.alloc(host.size());
-        s.far_mask.alloc((size_t)blocks * plan.words);
-        s.far_coef.alloc((size_t)blocks * kFarPoints * kFarPoints * kFarPoints);
+        try {
+            s.far_tables.alloc(host.size());
+            s.far_mask.alloc((size_t)blocks * plan.words);
+            s.far_coef.alloc((size_t)blocks * kFarPoints * kFarPoints * kFarPoints);
+        } catch (const Failure&) {   // no room beside the grid: the direct sum needs none
+            cudaGetLastError();
+            s.far_tables.release();
+            s.far_mask.release();
+            s.far_coef.release();
+            s.far_planned = true;
+            return;
+        }
         cuda_check(cudaMemcpyAsync(s.far_tables.p, host.data(), host.size(), cudaMemcpyHostToDevice, st),
                    "upload grid plan");
         cuda_check(cudaStreamSynchronize(st), "upload grid plan");

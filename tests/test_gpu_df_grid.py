@@ -16,7 +16,8 @@ pytestmark = pytest.mark.gpu
 
 
 def small_slab(**kw):
-    return synth.slab(nlx=6, nly=6, layers=3, cell=(12.0, 12.0, 20.0), zhigh=18.0, zlow=17.85, tip_charge=-0.02, **kw)
+    kw = {"zhigh": 18.0, "zlow": 17.85, **kw}
+    return synth.slab(nlx=6, nly=6, layers=3, cell=(12.0, 12.0, 20.0), tip_charge=-0.02, **kw)
 
 
 SPECS = {
@@ -38,6 +39,20 @@ def test_interpolated_build_matches_fp64(tmp_path, name):
     np.testing.assert_allclose(got["tip"], want["tip"], rtol=0, atol=1e-8)
     np.testing.assert_allclose(got["force"], want["force"], rtol=1e-8, atol=1e-8)
     np.testing.assert_allclose(got["energy"], want["energy"], rtol=1e-8, atol=1e-8)
+
+
+@pytest.mark.parametrize("lj,a", [(True, 1.5), (False, 1.5), (False, 3.0)])
+def test_weak_forces_keep_their_relative_accuracy(tmp_path, lj, a):
+    """The dummy 12 A above a slab of Morse and LJ or only Morse terms every force is small;
+    relative to itself it stays within 1e-9 of FP64 (a term's rounding is about
+    1e-13, a position's 1e-11 A times a)."""
+    spec = small_slab(pixels=76, step=0.2, external=False, zhigh=26.0, zlow=25.85)
+    spec.overwrites = [("O", t, "morse", 0.1, a, 3.2) for t in (("C",) if lj else ("C", "N"))]
+    scan = Scan(Input(spec.write(str(tmp_path))).desc(), device=0)
+    want, _ = scan.run(_abi.FP64)
+    got, _ = scan.run(_abi.DF)
+    np.testing.assert_array_equal(got["steps"], want["steps"])
+    np.testing.assert_allclose(got["force"][:, 2], want["force"][:, 2], rtol=1e-9, atol=0)
 
 
 def test_interpolated_rebuild_is_identical_and_can_be_captured(tmp_path):
