@@ -1527,9 +1527,8 @@ int mafm_autotune(mafm_scan* const* scans, int32_t n_scans, mafm_run_opts* best,
         struct EvGuard { cudaEvent_t a, b; ~EvGuard() { cudaEventDestroy(a); cudaEventDestroy(b); } } eg{e0, e1};
         // The sweep runs on the first kTrialScans scans of a batch; the winner
         // is then timed against the default shape on the whole batch (a
-        // subset of a large batch can favour another shape: 256 molecules,
-        // the first 32 favour G = 2 with 64-column tiles, all 256 G = 1 with
-        // 128-column tiles, 5 % faster).
+        // subset of a large batch can favour another shape, with more lanes a
+        // column and shorter tiles).
         constexpr int kTrialScans = 32;
         int n_time = std::min(n_scans, (int32_t)kTrialScans);
         auto time_opts = [&](const mafm_run_opts& o, bool warm = true) {
@@ -1557,8 +1556,7 @@ int mafm_autotune(mafm_scan* const* scans, int32_t n_scans, mafm_run_opts* best,
             o.lanes_per_column = G;
             // one scan: one-column tiles balance large scans, whole-warp tiles
             // keep a warp's lanes busy when there are fewer columns than
-            // groups; batches: one or four columns per group (longer tiles
-            // make the waits at scan boundaries rarer)
+            // groups; batches: one or four columns per group
             const int t_a = n_scans > 1 ? 32 / G : 1, t_b = n_scans > 1 ? 128 / G : 32 / G;
             for (int ti = 0; ti < (t_b == t_a ? 1 : 2); ++ti) {   // G = 32: one shape
                 o.columns_per_tile = ti == 0 ? t_a : t_b;
