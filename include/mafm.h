@@ -413,6 +413,11 @@ int mafm_scan_grid_info(const mafm_scan* scan, int32_t what, int32_t n[3],
                         double basis[9], double origin[3]);
 /* Copy the FP64 grid nodes {Fx,Fy,Fz,E} (n0*n1*n2*4 doubles, z fastest). */
 int mafm_scan_grid_copy(const mafm_scan* scan, int32_t what, double* out);
+/* The rigid grid that MAFM_DF runs read, built if it has not been: blocks (may
+ * be NULL) receives the blocks per axis between whose Chebyshev points the far
+ * terms were interpolated, 0, 0, 0 where every term was summed at every node;
+ * out (may be NULL) the nodes {Fx,Fy,Fz,E} as for mafm_scan_grid_copy. */
+int mafm_scan_grid_df(mafm_scan* scan, int32_t blocks[3], double* out);
 /* (Re)build the rigid force grid of a rigidgrid scan for one precision on the
  * stream: Simulation::buildTipGridInteractions (simulation.cpp:420-501), which
  * the reference runs once per scan before the pixel loop.  mafm_run builds the

@@ -952,9 +952,16 @@ __global__ void nodes_df_to_64_kernel(const NodeDF* in, Node64* out, long long n
 // to the block's nodes, and only the records near the block are evaluated at every
 // node.  A record is far from a block when, on every axis, the ellipse around the
 // block's interval (scaled to [-1, 1]) on which the term has its nearest
-// singularity has a half axis of at least kFarAxis: a term (r^-1 to r^-14) is then
-// interpolated to 1e-15 of itself or better (the r^-14 part, which converges
-// slowest, is below 1e-4 of its r^-7 part there).  Morse records are always near:
+// singularity has a half axis of at least kFarAxis.  At that distance a force
+// r^-7 is interpolated to 4.2e-16 of itself at worst, the Coulomb force and an
+// energy r^-6 better, and a force r^-13 to 3.1e-13 beside a block much longer than
+// wide, 6e-14 beside a block about as long as wide (evaluated in extended
+// precision; 1.3e-14 from 12 on, 1e-15 from 14 on).  That part is at most 2 (sigma /
+// r)^6 of a term's force, with r >= 7.2 A for the shortest blocks (1.6 A) and 14.4 A
+// for 3.2 A ones, so that for sigma = 3.2 A a term is good to 5e-15 and 5e-16 of itself.  What a
+// double-float term itself rounds is larger: nodes above slabs and molecules
+// differ from the FP64 build by 4e-14 to 1e-13 rms with either build, also where the
+// pairs have no attraction at all (up to 7e-13 at single nodes).  Morse records are always near:
 // exp(-2 a r) over an interval of half length h converges with a h, whatever the
 // distance, and a term with a = 2 A^-1 over 3.2 A would be good to 1e-7 of itself
 // only, which counts where every term is weak.  Blocks, Chebyshev points and the

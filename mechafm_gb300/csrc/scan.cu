@@ -1288,6 +1288,20 @@ int mafm_scan_grid_copy(const mafm_scan* scan, int32_t what, double* out) {
     });
 }
 
+int mafm_scan_grid_df(mafm_scan* scan, int32_t blocks[3], double* out) {
+    return guarded([&] {
+        if (!scan) fail(MAFM_E_INVALID, "null scan");
+        if (!scan->d.rigidgrid) fail(MAFM_E_INVALID, "the scan has no rigid grid");
+        cuda_check(cudaSetDevice(scan->device), "cudaSetDevice");
+        ensure_grid_df(*scan, nullptr);
+        if (blocks)
+            for (int a = 0; a < 3; ++a) blocks[a] = scan->far_used ? scan->far.nb[a] : 0;
+        if (!out) return;
+        const size_t N = (size_t)scan->grid_view.n[0] * scan->grid_view.n[1] * scan->grid_view.n[2];
+        cuda_check(cudaMemcpy(out, scan->griddf64.p, N * sizeof(Node64), cudaMemcpyDeviceToHost), "download grid");
+    });
+}
+
 }  // extern "C"
 
 namespace mafm {

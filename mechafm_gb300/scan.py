@@ -286,6 +286,15 @@ class Scan:
         check(lib().mafm_scan_grid_copy(self._h, what, ptr(out)))
         return out.reshape(n[0], n[1], n[2], 4)
 
+    def grid_df(self):
+        """The nodes MAFM_DF runs read, and the blocks per axis of their build
+        (zeros: every term at every node)."""
+        n, _, _ = self.grid_info()
+        out = np.zeros(n[0] * n[1] * n[2] * 4)
+        blocks = (C.c_int32 * 3)()
+        check(lib().mafm_scan_grid_df(self._h, blocks, ptr(out)))
+        return out.reshape(n[0], n[1], n[2], 4), tuple(blocks)
+
 
 def run_batch(scans: list, precision=_abi.FP32C, lanes=0, block=0, tile=0, stream=None):
     """Relax several scans in one persistent launch; returns (list of points, stats)."""
