@@ -391,13 +391,24 @@ int mafm_df_weights(const mafm_df_params* params, double dz, double* w, int32_t 
 /* df[s][x][y] for every window s of n_w heights (nz - n_w windows, ascending
  * z): fz[((x*ny + y)*nz + k) * stride] is Fz at scan level k (k = 0 at zhigh);
  * stride 8 reads mafm_point.force[2] (pass &pts[0].force[2]).  Host or device
- * memory; with device memory on both sides the call is ordered on the stream
- * and returns without waiting (as mafm_run with device output). */
+ * memory; the images are complete when the call returns. */
 int mafm_df(const double* fz, int64_t stride, int32_t nx, int32_t ny, int32_t nz, double dz,
             const mafm_df_params* params, double* df, void* stream);
 /* Transpose of mafm_df: dL/dFz (nx*ny*nz, level order) from dL/ddf. */
 int mafm_df_adjoint(const double* g_df, int32_t nx, int32_t ny, int32_t nz, double dz,
                     const mafm_df_params* params, double* g_fz, void* stream);
+/* The same two, ordered on the stream: with device memory on both sides the
+ * result may be complete only when the stream gets there, so a reader on
+ * another stream (or the host) waits for an event of this one, and the buffers
+ * stay valid until then.  They return without waiting, allocate nothing and can
+ * be captured while the window has at most 128 weights and 32 columns of the
+ * stacks fit 48 KB (nz up to 191; for the transpose nz plus the number of windows
+ * up to 191); otherwise, and with host or managed memory, they wait like the
+ * calls above. */
+int mafm_df_async(const double* fz, int64_t stride, int32_t nx, int32_t ny, int32_t nz, double dz,
+                  const mafm_df_params* params, double* df, void* stream);
+int mafm_df_adjoint_async(const double* g_df, int32_t nx, int32_t ny, int32_t nz, double dz,
+                          const mafm_df_params* params, double* g_fz, void* stream);
 
 /* Evaluate the tip–surface force and energy at n given tip positions
  * (System::evalTipSurfaceForces, system.cpp:41-51): pairs, external field or

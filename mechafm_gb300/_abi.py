@@ -143,6 +143,10 @@ SIGNATURES = {
                           C.POINTER(DfParams), _P, _P]),
     "mafm_df_adjoint": (C.c_int, [_P, C.c_int32, C.c_int32, C.c_int32, C.c_double,
                                   C.POINTER(DfParams), _P, _P]),
+    "mafm_df_async": (C.c_int, [_P, C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_double,
+                                C.POINTER(DfParams), _P, _P]),
+    "mafm_df_adjoint_async": (C.c_int, [_P, C.c_int32, C.c_int32, C.c_int32, C.c_double,
+                                        C.POINTER(DfParams), _P, _P]),
     "mafm_scan_sample": (C.c_int, [_P, C.c_int32, C.c_int32, _P, C.c_int64, _P]),
     "mafm_scan_grid_info": (C.c_int, [_P, C.c_int32, C.c_int32 * 3, C.c_double * 9,
                                       C.c_double * 3]),

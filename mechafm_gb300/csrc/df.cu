@@ -84,9 +84,9 @@ struct InlineW {
 // (transpose); one thread per value with the stack read in place took 90.5
 // and 105 us.  What bounds them is the FP64 pipe: one FMA per weight and value,
 // 4.2e7 of them at that size, and an SM takes a warp's FMA every 19 cycles.
-// The whole pass, images and gradient from Python, went from 852 to 211 us
-// there and from 654 to 212 us at 64 x 64 x 41: two allocations, two frees
-// and a wait of each call are gone.
+// The whole pass, images and gradient from Python (stream-ordered calls), went from
+// 852 to 211 us there and from 654 to 212 us at 64 x 64 x 41: two allocations, two
+// frees and a wait of each call are gone.
 constexpr int kTileXY = 32;
 constexpr int kTileThreads = 256;
 
@@ -230,8 +230,8 @@ extern "C" int mafm_df_weights(const mafm_df_params* params, double dz, double* 
     });
 }
 
-// Shared by mafm_df and mafm_df_adjoint: host or device buffers, one stream.
-static int df_apply(bool adjoint, const double* in, int64_t stride, int32_t nx, int32_t ny, int32_t nz,
+// Host or device buffers, one stream.  wait: the result is complete on return.
+static int df_apply(bool wait, bool adjoint, const double* in, int64_t stride, int32_t nx, int32_t ny, int32_t nz,
                     double dz, const mafm_df_params* params, double* out, void* stream) {
     return guarded([&] {
         if (!in || !out || nx < 1 || ny < 1 || nz < 1) fail(MAFM_E_INVALID, "bad df arguments");
@@ -289,19 +289,29 @@ static int df_apply(bool adjoint, const double* in, int64_t stride, int32_t nx, 
         cuda_check(cudaGetLastError(), "df launch");
         if (host_out)
             cuda_check(cudaMemcpyAsync(out, dst, (size_t)n_out * sizeof(double), cudaMemcpyDeviceToHost, st), "download");
-        // Device memory in and out: the call is stream-ordered and does not
-        // wait.  Host (and managed) results are complete on return, and buffers
-        // of this call are freed only when the stream is done with them.
-        if (!frees.p.empty() || host_readable(in) || host_readable(out)) cuda_check(cudaStreamSynchronize(st), "df");
+        // A stream-ordered call waits all the same where host (or managed) memory
+        // takes part, and before buffers of its own are freed.
+        if (wait || !frees.p.empty() || host_readable(in) || host_readable(out))
+            cuda_check(cudaStreamSynchronize(st), "df");
     });
 }
 
 extern "C" int mafm_df(const double* fz, int64_t stride, int32_t nx, int32_t ny, int32_t nz, double dz,
                        const mafm_df_params* params, double* df, void* stream) {
-    return df_apply(false, fz, stride, nx, ny, nz, dz, params, df, stream);
+    return df_apply(true, false, fz, stride, nx, ny, nz, dz, params, df, stream);
 }
 
 extern "C" int mafm_df_adjoint(const double* g_df, int32_t nx, int32_t ny, int32_t nz, double dz,
                                const mafm_df_params* params, double* g_fz, void* stream) {
-    return df_apply(true, g_df, 1, nx, ny, nz, dz, params, g_fz, stream);
+    return df_apply(true, true, g_df, 1, nx, ny, nz, dz, params, g_fz, stream);
+}
+
+extern "C" int mafm_df_async(const double* fz, int64_t stride, int32_t nx, int32_t ny, int32_t nz, double dz,
+                             const mafm_df_params* params, double* df, void* stream) {
+    return df_apply(false, false, fz, stride, nx, ny, nz, dz, params, df, stream);
+}
+
+extern "C" int mafm_df_adjoint_async(const double* g_df, int32_t nx, int32_t ny, int32_t nz, double dz,
+                                     const mafm_df_params* params, double* g_fz, void* stream) {
+    return df_apply(false, true, g_df, 1, nx, ny, nz, dz, params, g_fz, stream);
 }

@@ -85,18 +85,21 @@ def _torch_df(fz, dz, prm, adjoint):
     x = fz.detach().contiguous().double()
     nx, ny = x.shape[-2:] if adjoint else x.shape[:2]
     pp = C.byref(prm) if prm is not None else None
-    stream = C.c_void_p(torch.cuda.current_stream(x.device).cuda_stream) if x.is_cuda else None
+    stream = None
+    if x.is_cuda:   # ordered on the current stream, as torch's own operators are
+        current = torch.cuda.current_stream(x.device)
+        stream = C.c_void_p(current.cuda_stream)
     if adjoint:
         nz = adjoint
         out = torch.empty((nx, ny, nz), dtype=torch.float64, device=x.device)
-        check(lib().mafm_df_adjoint(C.c_void_p(x.data_ptr()), nx, ny, nz, dz, pp,
-                                    C.c_void_p(out.data_ptr()), stream))
+        check(lib().mafm_df_adjoint_async(C.c_void_p(x.data_ptr()), nx, ny, nz, dz, pp,
+                                          C.c_void_p(out.data_ptr()), stream))
     else:
         nz = x.shape[2]
         nw = _n_weights(dz, prm)
         out = torch.empty((max(nz - nw, 0), nx, ny), dtype=torch.float64, device=x.device)
-        check(lib().mafm_df(C.c_void_p(x.data_ptr()), 1, nx, ny, nz, dz, pp,
-                            C.c_void_p(out.data_ptr()), stream))
+        check(lib().mafm_df_async(C.c_void_p(x.data_ptr()), 1, nx, ny, nz, dz, pp,
+                                  C.c_void_p(out.data_ptr()), stream))
     return out
 
 

@@ -153,3 +153,41 @@ def test_df_tiles_match_oracle(nx, ny, nz, dz):
     pts = np.zeros(fz.size, dtype=_abi.POINT_DTYPE)
     pts["force"][:, 2] = fz.reshape(-1)
     np.testing.assert_array_equal(df.df_images(pts, dz, shape=fz.shape), img.detach().cpu().numpy())
+
+
+def _rounding(dz, x):
+    """A window's FP64 rounding: n terms of 2^-53 of the largest partial sum, with room of 4."""
+    w, fac = odf.weights(dz)
+    return 4 * len(w) * 2.0 ** -53 * fac * dz * np.abs(w).sum() * np.abs(x).max()
+
+
+@pytest.mark.gpu
+def test_df_calls_and_other_streams():
+    """mafm_df and mafm_df_adjoint return when their device results are there; the
+    stream-ordered calls return before, and their results hold for a reader that
+    waits for an event (the stream is busy for some 50 ms before each call)."""
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+    nx, ny, nz, dz = 64, 33, 24, 0.1
+    fz = torch.tensor(_stack(11, nx, ny, nz), device="cuda")
+    nw = len(df.weights(dz)[0])
+    g = torch.randn(nz - nw, nx, ny, dtype=torch.float64, device="cuda")
+    want = {"mafm_df": odf.df_images(fz.cpu().numpy(), dz), "mafm_df_adjoint": odf.df_adjoint(g.cpu().numpy(), nz, dz)}
+    x = fz.clone().requires_grad_(True)
+    df.df_image_torch(x, dz).backward(g)   # a kernel's first launch may wait for the device by itself
+    side = torch.cuda.Stream()
+    for name, x in (("mafm_df", fz), ("mafm_df_adjoint", g)):
+        stride = () if name.endswith("adjoint") else (1,)
+        for suffix in ("", "_async"):
+            out = torch.zeros(want[name].shape, dtype=torch.float64, device="cuda")
+            torch.cuda.synchronize()
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(100_000_000)
+            call = getattr(_abi.lib(), name + suffix)
+            _abi.check(call(C.c_void_p(x.data_ptr()), *stride, nx, ny, nz, dz, None, C.c_void_p(out.data_ptr()),
+                            C.c_void_p(side.cuda_stream)))
+            assert side.query() == (suffix == "")
+            if suffix:
+                torch.cuda.current_stream().wait_event(side.record_event())
+            got = out.cpu().numpy()
+            np.testing.assert_allclose(got, want[name], rtol=0, atol=_rounding(dz, x.cpu().numpy()))
