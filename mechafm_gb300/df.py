@@ -88,6 +88,7 @@ def _torch_df(fz, dz, prm, adjoint):
     stream = None
     if x.is_cuda:   # ordered on the current stream, as torch's own operators are
         current = torch.cuda.current_stream(x.device)
+        x.record_stream(current)   # x may be of another stream and freed before this one gets there
         stream = C.c_void_p(current.cuda_stream)
     if adjoint:
         nz = adjoint

@@ -191,3 +191,23 @@ def test_df_calls_and_other_streams():
                 torch.cuda.current_stream().wait_event(side.record_event())
             got = out.cpu().numpy()
             np.testing.assert_allclose(got, want[name], rtol=0, atol=_rounding(dz, x.cpu().numpy()))
+
+
+@pytest.mark.gpu
+def test_df_image_of_a_freed_tensor_of_another_stream():
+    """The stack may be freed, and its memory taken again on its own stream, before
+    the stream of the images gets to it."""
+    torch = pytest.importorskip("torch")
+    data = _stack(12, 64, 64, 24)
+    want = odf.df_images(data, 0.1)
+    side = torch.cuda.Stream()
+    fz = torch.tensor(data, device="cuda")
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(100_000_000)
+        img = df.df_image_torch(fz, 0.1)
+    del fz
+    for _ in range(4):
+        torch.full(data.shape, 1e30, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    np.testing.assert_allclose(img.cpu().numpy(), want, rtol=0, atol=_rounding(0.1, data))
