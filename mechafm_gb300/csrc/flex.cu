@@ -45,6 +45,7 @@ struct mafm_flex {
         const double* dihedral_par;
         const int* pairs;           // [2 n_pairs]
         const void* pair_par;       // FlexPair[n_pairs]
+        const void* coul;           // FlexCoul of the pairs with charges
         const double* xy;           // [3 n_xy] atom (as double), x0, y0
         const int* list_begin;      // [n_sys + 1]
         const int* list;            // per atom, in the reference's order: slot << 1 | negated
@@ -55,8 +56,6 @@ struct mafm_flex {
         int n_energies;             // the tip's terms: slots 0 .. n_energies - 1
     } dv{};
     int n_slots = 0;
-    double* scratch = nullptr;      // energies and slots of every block, when shared memory is too small
-    size_t scratch_doubles = 0;
     mafm::RunCounters* ctr = nullptr;
     mafm::RunCounters* host_ctr = nullptr;
     double sub[6] = {0, 0, 0, 0, 0, 0};   // multiplier, ulj, ushift, z0, rc, sig
@@ -89,10 +88,13 @@ struct FlexTS {          // one tip–surface term: LJ / Morse (+ the image shif
     int pad;
 };
 
-struct FlexPair {        // one non-bonded surface pair
-    int kind;
-    int pad;
+struct FlexPair {        // van der Waals part of a non-bonded pair
+    int kind, pad;
     double p[3];
+};
+
+struct FlexCoul {        // Coulomb part of one whose charges are not zero
+    int i, j;
     double qq;
 };
 
@@ -268,8 +270,8 @@ __device__ void eval_task(const FlexKernelArgs& A, const double* pe, int kind, i
             break;
         }
         case FT_PAIR_COUL: {
-            const int i = dv.pairs[2 * idx], j = dv.pairs[2 * idx + 1];
-            put3(res, slot, coul_force(pp[idx].qq, sub3(P3(i), P3(j)), e));
+            const FlexCoul& q = static_cast<const FlexCoul*>(dv.coul)[idx];
+            put3(res, slot, coul_force(q.qq, sub3(P3(q.i), P3(q.j)), e));
             break;
         }
         case FT_SUBSTRATE: { // SubstrateInteraction (interactions.cpp:280-296); idx: the atom
@@ -760,7 +762,6 @@ extern "C" int mafm_flex_create(int device, const mafm_scan_desc* d, const mafm_
                 FlexPair x{};
                 x.kind = f->pair_vdw[q].kind;
                 for (int k = 0; k < 3; ++k) x.p[k] = f->pair_vdw[q].p[k];
-                x.qq = f->pair_qq ? f->pair_qq[q] : 0.0;
                 pp.push_back(x);
             }
             for (int a : bonds)
@@ -782,12 +783,15 @@ extern "C" int mafm_flex_create(int device, const mafm_scan_desc* d, const mafm_
             }
             for (int g = 0; g < f->n_dihedrals; ++g)
                 for (int r = 0; r < 4; ++r) add(dihedrals[4 * g + r], FT_DIHEDRAL, r, g);
+            std::vector<FlexCoul> coul;
             for (int q = 0; q < f->n_pairs; ++q) {
                 add(pairs[2 * q], FT_PAIR_VDW, 0, q);
                 add(pairs[2 * q + 1], FT_PAIR_VDW, 1, q);
-                if (pp[q].qq != 0) {
-                    add(pairs[2 * q], FT_PAIR_COUL, 0, q);
-                    add(pairs[2 * q + 1], FT_PAIR_COUL, 1, q);
+                if (f->pair_qq && f->pair_qq[q] != 0) {
+                    const int c = (int)coul.size();
+                    coul.push_back({pairs[2 * q], pairs[2 * q + 1], f->pair_qq[q]});
+                    add(pairs[2 * q], FT_PAIR_COUL, 0, c);
+                    add(pairs[2 * q + 1], FT_PAIR_COUL, 1, c);
                 }
             }
             // buildSubstrateInteractions (simulation.cpp:516-528)
@@ -813,7 +817,7 @@ extern "C" int mafm_flex_create(int device, const mafm_scan_desc* d, const mafm_
             // tip–surface terms index one list)
             const int n_ts = (int)ts.size();
             const int count[12] = {0, n_ts, 1, 1, 1, f->n_bonds, f->n_angles, f->n_dihedrals,
-                                   f->n_pairs, f->n_pairs, na, (int)xy.size() / 3};
+                                   f->n_pairs, (int)coul.size(), na, (int)xy.size() / 3};
             int slots = 0;
             for (int kd = FT_TS_VDW; kd <= FT_XY; ++kd) {
                 s->dv.slot_base[kd] = slots;
@@ -882,6 +886,7 @@ extern "C" int mafm_flex_create(int device, const mafm_scan_desc* d, const mafm_
             const size_t o_dp = piece(f->dihedral_param, (size_t)f->n_dihedrals * 2 * sizeof(double));
             const size_t o_pr = piece(pairs.data(), pairs.size() * sizeof(int));
             const size_t o_pp = piece(pp.data(), pp.size() * sizeof(FlexPair));
+            const size_t o_cp = piece(coul.data(), coul.size() * sizeof(FlexCoul));
             const size_t o_xy = piece(xy.data(), xy.size() * sizeof(double));
             const size_t o_lb = piece(begin.data(), begin.size() * sizeof(int));
             const size_t o_l = piece(list.data(), list.size() * sizeof(int));
@@ -905,6 +910,7 @@ extern "C" int mafm_flex_create(int device, const mafm_scan_desc* d, const mafm_
             s->dv.dihedral_par = reinterpret_cast<const double*>(dev + o_dp);
             s->dv.pairs = reinterpret_cast<const int*>(dev + o_pr);
             s->dv.pair_par = dev + o_pp;
+            s->dv.coul = dev + o_cp;
             s->dv.xy = reinterpret_cast<const double*>(dev + o_xy);
             s->dv.list_begin = reinterpret_cast<const int*>(dev + o_lb);
             s->dv.list = reinterpret_cast<const int*>(dev + o_l);
@@ -928,7 +934,6 @@ extern "C" int mafm_flex_destroy(mafm_flex* s) {
     if (s) {
         cudaSetDevice(s->device);
         if (s->dev_block) cudaFree(s->dev_block);
-        if (s->scratch) cudaFree(s->scratch);
         if (s->ctr) cudaFree(s->ctr);
         if (s->host_ctr) cudaFreeHost(s->host_ctr);
         delete s;
@@ -967,9 +972,11 @@ extern "C" int mafm_flex_run(mafm_flex* s, int32_t col_begin, int32_t col_end, m
         struct Frees {
             void* a = nullptr;
             void* b = nullptr;
+            double* scratch = nullptr;
             ~Frees() {
                 if (a) cudaFree(a);
                 if (b) cudaFree(b);
+                if (scratch) cudaFree(scratch);
             }
         } frees;
         if (void* v = device_view(out)) {
@@ -1017,15 +1024,21 @@ extern "C" int mafm_flex_run(mafm_flex* s, int32_t col_begin, int32_t col_end, m
         cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, flex_kernel, 32 * kFlexWarps, smem),
                    "flex occupancy");
         const int cols = col_end - col_begin;
-        const int blocks = std::max(1, std::min(cols, sm_count() * (in_smem ? std::max(per_sm, 1) : 1)));
-        if (!in_smem && blocks * block_doubles > s->scratch_doubles) {
-            if (s->scratch) cudaFree(s->scratch);
-            s->scratch = nullptr;
-            s->scratch_doubles = 0;
-            cuda_check(cudaMalloc(&s->scratch, blocks * block_doubles * sizeof(double)), "cudaMalloc");
-            s->scratch_doubles = blocks * block_doubles;
+        int blocks = std::max(1, std::min(cols, sm_count() * (in_smem ? std::max(per_sm, 1) : 1)));
+        if (!in_smem) {
+            // Slots of this call, 24 B each and a set per block: 12 MB a block (25 MB
+            // with charges) for the 520,000 pairs of 1,022 atoms in small fragments.
+            // They are given back when the call ends, and where they do not fit
+            // fewer blocks take the columns.
+            cudaError_t e;
+            while ((e = cudaMalloc(&frees.scratch, blocks * block_doubles * sizeof(double))) ==
+                       cudaErrorMemoryAllocation && blocks > 1) {
+                cudaGetLastError();
+                blocks /= 2;
+            }
+            cuda_check(e, "cudaMalloc");
         }
-        A.scratch = in_smem ? nullptr : s->scratch;
+        A.scratch = frees.scratch;
         if (cols > 0) {
             flex_kernel<<<blocks, 32 * kFlexWarps, smem, st>>>(A);
             cuda_check(cudaGetLastError(), "flex launch");

@@ -130,3 +130,26 @@ def test_gpu_sizes_match_oracle(tmp_path, n_h2, opt):
     np.testing.assert_allclose(pts["tip"], want["tip"], rtol=0, atol=1e-6)
     np.testing.assert_allclose(pts["force"], want["force"], rtol=1e-6, atol=1e-9)
     np.testing.assert_allclose(states, want_states, rtol=0, atol=1e-6)
+
+
+@pytest.mark.gpu
+def test_gpu_workspace_is_given_back(tmp_path):
+    """Force slots past shared memory live in device memory during a call only,
+    and pairs without charges need none for a Coulomb term."""
+    torch = pytest.importorskip("torch")
+    _, desc, flex = _with_hydrogens(tmp_path, 60, maxsteps="30")
+    neutral = np.zeros(flex.c.n_pairs)
+    neutral[::3] = np.ctypeslib.as_array(flex.c.pair_qq, shape=neutral.shape)[::3]
+    flex.c.pair_qq = neutral.ctypes.data_as(type(flex.c.pair_qq))
+    warm = FlexScan(desc, flex, device=0)
+    warm.run()                       # the first launch loads the kernel
+    warm.close()
+    torch.cuda.synchronize()
+    scan = FlexScan(desc, flex, device=0)
+    free = torch.cuda.mem_get_info()[0]
+    pts, _, _ = scan.run()
+    assert torch.cuda.mem_get_info()[0] == free
+    want, _, _ = oracle.flex_run(desc, flex)
+    np.testing.assert_array_equal(pts["steps"], want["steps"])
+    np.testing.assert_allclose(pts["tip"], want["tip"], rtol=0, atol=1e-6)
+    np.testing.assert_allclose(pts["force"], want["force"], rtol=1e-6, atol=1e-9)
