@@ -463,11 +463,19 @@ __device__ __forceinline__ void tip_dummy_df(const ScanParamsDF& p, VecDF<G> tip
 
 enum : int { DF_EVAL0 = 0, DF_EVAL1 = 1, DF_EVAL2 = 2, DF_EVAL3 = 3, DF_OUT = 4 };
 
+// Steps of a height up to which its lane does not wait for the warp's stage.  300 x
+// 300 cluster x 15 heights that converge in energy after a few steps: rk4 4.33 ms,
+// with waiting 5.21, midpoint 2.46 / 2.68; force and energy, hundreds of steps: the
+// same either way (rk4 126 ms, never waiting 131-137; 101 x 101 graphene 103, never
+// waiting 113-115).  4 and 16 measure the same as 8.
+constexpr int kAlignSteps = 8;
+
 // One lane's column: the state fire_t / sd_t keep in locals, held across
 // slots.  u is the midpoint v2 / the RK4 v_k; vs, fs, es the RK4 sums.
 template <int G>
 struct LaneDF {
     int col, scan, k, n, nnn, phase, tie, outside;
+    bool aligned;   // waits for the warp's stage
     VecDF<G> tip, vel, dum, ex, u, vs, fs;
     D energy, es, alpha, dt;
 };
@@ -622,6 +630,7 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
                     s.energy = D(0);
                     s.k = 0;
                     s.tie = 0;
+                    s.aligned = true;
                     start_level();
                 }
             }
@@ -637,10 +646,10 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
         // iteration (midpoint; rk4: every fourth), so that the lanes of a warp
         // are in the same stage: without it they drift apart by one evaluation
         // at every record, and the warp runs every stage's code in every
-        // iteration.  A lane waits for at most one (three) of a height's
-        // hundreds of evaluations (401 x 401 cluster 627 -> 599 ms, 101 x 101
-        // graphene 115 -> 107 ms).
-        if ((s.phase == DF_EVAL0 || s.phase == DF_OUT) && (ticks & P.stage_mask)) continue;
+        // iteration.  A lane waits for at most one (three) evaluations of a
+        // height, so heights of few steps are not worth it: a lane whose last
+        // height took kAlignSteps or fewer does not wait.
+        if (s.aligned && (s.phase == DF_EVAL0 || s.phase == DF_OUT) && (ticks & P.stage_mask)) continue;
 
         // ---- one evaluation per lane ----
         VecDF<G> F;
@@ -678,6 +687,7 @@ __global__ void __launch_bounds__(128) relaxdf_kernel(const BatchDF* __restrict_
                 s.dum.z = s.dum.z - P.dz;
                 s.tip.z = s.tip.z - P.dz;
             }
+            s.aligned = s.n > kAlignSteps;
             if (++s.k < P.nz) {
                 start_level();
             } else {
