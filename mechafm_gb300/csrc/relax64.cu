@@ -1,8 +1,9 @@
 // relax64.cu — the plain FP64 GPU path (precision MAFM_FP64).
 //
-// A group of 4 to 32 lanes of a warp per pixel column, columns handed out by a
-// global atomic counter.  Every floating-point expression keeps the reference's operation order and
-// this translation unit is compiled with -fmad=false, so no a*b+c is fused:
+// A group of 4 to 32 lanes of a warp per pixel column (one thread where columns
+// are many and terms few), columns handed out by a global atomic counter.  Every
+// floating-point expression keeps the reference's operation order and this
+// translation unit is compiled with -fmad=false, so no a*b+c is fused:
 // with LJ and Coulomb terms the results are bit-identical to the reference's
 // x86-64 build (division and square root are correctly rounded in both; exp
 // in the Morse term may differ in the last bit).
@@ -463,6 +464,31 @@ __global__ void __launch_bounds__(32 * W) relax64_kernel(const __grid_constant__
     }
 }
 
+// One thread a column: the same bits, for so many columns that they fill the GPU by
+// themselves and evaluations of so few terms that the rest of a step, which a quad's
+// lanes repeat, is most of the work (thread_per_column).
+__global__ void __launch_bounds__(128) relax64_thread_kernel(const __grid_constant__ ScanParams p, mafm_point* out,
+                                                             RunCounters* ctr, const int* list, int col_begin,
+                                                             long long n_cols, bool by_column, int smem_cap) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const AtomRec64* atoms = stage64(p, reinterpret_cast<AtomRec64*>(smem_raw), smem_cap);
+    Eval64 ev{p, atoms, p.n_terms_direct, p.ts_mode, 0u, 0ull};
+    long long steps = 0;
+    unsigned long long evals = 0;
+    unsigned status_or = 0;
+    for (;;) {
+        const long long w = (long long)atomicAdd(&ctr->next_work, 1ull);
+        if (w >= n_cols) break;
+        const int col = list ? list[w] : col_begin + (int)w;
+        relax_column_t<double>(ev, p, col, out + (by_column ? (size_t)(col - col_begin) : (size_t)w) * p.nz, true,
+                               false, steps, evals, status_or);
+    }
+    atomicAdd(&ctr->total_steps, (unsigned long long)steps);
+    atomicAdd(&ctr->force_evals, evals);
+    atomicAdd(&ctr->pair_evals, ev.pairs);
+    if (status_or | ev.err) atomicOr(&ctr->error_word, status_or | ev.err);
+}
+
 // FP64 re-relaxation of the double-float kernel's near-tie columns (scan << 32 |
 // column), one warp per column.  Persistent: each warp takes the next listed
 // column and relaxes it from its top height with EvalWarp64, which forms every
@@ -573,6 +599,39 @@ static cudaError_t launch_relax64_g(const ScanParams& p, mafm_point* out, RunCou
     return cudaGetLastError();
 }
 
+// Whether a thread a column is faster than four lanes a column.  The lanes share the
+// terms but repeat the rest of an evaluation, so the fewer terms, the fewer columns
+// it takes; the in-order sums of Coulomb records leave lanes idle and a field's lookup
+// is not shared, so that such scans change over earlier.  Two heights of a scan, one thread / lanes, ms:
+//   rigid grid  6,400 columns 2.92 / 2.46, 10,000 2.92 / 3.52, 160,000 22.6 / 48.7
+//   field and 16 terms  10,000 9.3 / 7.2, 22,500 11.4 / 18.0
+//   LJ + Coulomb, 4 terms  8,100 5.2 / 4.9, 16,900 5.7 / 7.9; 20 terms  16,900 28.9 /
+//     24.3, 40,000 50.5 / 61.0; 60 terms  40,000 141 / 152, 176,000 473 / 579
+//   LJ  10 terms  16,900 5.4 / 6.1; 20 terms  16,900 12.4 / 11.3, 40,000 22.6 / 26.0;
+//     60 terms  40,000 72 / 66, 176,000 203 / 201
+// (4 LJ terms are an exception between 40,000 and 90,000 columns, 3.6 / 3.1 and 3.9 /
+// 3.4: a few long columns are what lasts.)
+static bool thread_per_column(const ScanParams& p, long long n_cols) {
+    const long long terms = p.ts_mode == 2 ? 0 : p.n_terms_direct;
+    return n_cols >= sm_count() * (45 + (p.has_coulomb || p.ts_mode == 1 ? 4 : 10) * terms);
+}
+
+static cudaError_t launch_relax64_thread(const ScanParams& p, mafm_point* out, RunCounters* ctr, const int* list,
+                                         int col_begin, long long n_cols, bool by_column, cudaStream_t s) {
+    int cap = 0, per_sm = 0;
+    const size_t smem = smem_bytes64(p, cap);
+    // One warp a block spreads the columns over the SMs (20 terms, 40,000 columns: 59.5
+    // -> 50.5 ms); more where every block's copy of the terms would fill the SM.
+    const int threads = smem <= 8 * 1024 ? 32 : 128;
+    cudaError_t e = cudaFuncSetAttribute(relax64_thread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, relax64_thread_kernel, threads, smem);
+    if (e != cudaSuccess) return e;
+    const long long blocks = std::min((n_cols + threads - 1) / threads, (long long)sm_count() * std::max(per_sm, 1));
+    relax64_thread_kernel<<<(unsigned)blocks, threads, smem, s>>>(p, out, ctr, list, col_begin, n_cols, by_column, cap);
+    return cudaGetLastError();
+}
+
 // Lanes per column: the fewest that give every SM four warps (an SM starts an
 // FP64 instruction every 19 cycles and a warp one every 64).  Four lanes cost
 // no more FP64 instructions per column than one, 8 / 16 / 32 lanes 9 / 38 / 95 %
@@ -587,6 +646,8 @@ cudaError_t launch_relax64(const ScanParams& p, mafm_point* out, RunCounters* ct
                            int col_begin, long long n_cols, int pairs_per_eval, bool by_column,
                            cudaStream_t s) {
     if (n_cols <= 0) return cudaSuccess;
+    if (thread_per_column(p, n_cols))
+        return launch_relax64_thread(p, out, ctr, list, col_begin, n_cols, by_column, s);
     int G = 4;
     while (G < 32 && n_cols * G < 32ll * 4 * sm_count()) G *= 2;
     const long long wide_cols = (p.has_coulomb ? 7ll : 4ll) * sm_count();
