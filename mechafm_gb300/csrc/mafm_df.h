@@ -107,6 +107,9 @@ cudaError_t launch_nodes_to_df(const Node64* in, NodeDF* out, long long n, cudaS
 // ---- the rigid grid's build with interpolated far terms (relaxdf.cu) ----
 constexpr int kFarPoints = 16;       // Chebyshev points per axis and block
 constexpr int kFarMaxNodes = 40;     // nodes per axis and block
+// Blocks built at a time: the coefficients of 512 take 67 MB, and their sums
+// still fill the GPU several times over.
+constexpr int kFarChunk = 512;
 // Half axis of the smallest ellipse of analyticity a far term has on every axis
 // (the block's interval being [-1, 1]): 10 means a convergence rate of 20 per point.
 constexpr float kFarAxis = 10.0f;
@@ -132,8 +135,9 @@ struct FarViewDF {
     const dfloat* lag[3];
     const float2* box[3];
     int words, max_strips, max_planes;
-    unsigned* mask;                  // words per block
-    NodeDF* coef;                    // kFarPoints^3 per block
+    int first;                       // block of a launch's first
+    unsigned* mask;                  // words per block of a launch
+    NodeDF* coef;                    // kFarPoints^3 per block of a launch
 };
 bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float>& xyz, int n_lj,
                  FarPlanDF& plan);

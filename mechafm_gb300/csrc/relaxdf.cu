@@ -1009,7 +1009,9 @@ struct FarBlock {
     int b[3];        // block index per axis
 };
 
-__device__ __forceinline__ FarBlock far_block(const FarViewDF& f, int id) {
+// Block at of a launch.
+__device__ __forceinline__ FarBlock far_block(const FarViewDF& f, int at) {
+    const int id = f.first + at;
     FarBlock q;
     q.b[2] = id % f.nb[2];
     q.b[1] = id / f.nb[2] % f.nb[1];
@@ -1393,7 +1395,7 @@ bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float
             blocks *= (double)bg[a].size() - 1;
         }
         const double coef = blocks * kFarP * kFarP * kFarP;
-        if (blocks > 65535 || coef * sizeof(NodeDF) > 8e9 || coef * n_rec > best) continue;
+        if (blocks > 65535 || coef * n_rec > best) continue;
         // near records, of a few blocks and at most about 1,000 records
         double near = 0;
         long long tried = 0;
@@ -1461,19 +1463,23 @@ bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float
 }
 
 static cudaError_t launch_far(const ScanParamsDF& p, NodeDF* out, Node64* out64, const FarViewDF& f, cudaStream_t s) {
-    const unsigned blocks = (unsigned)((long long)f.nb[0] * f.nb[1] * f.nb[2]);
-    far_classify_kernel<<<blocks, 128, 0, s>>>(f, p.pairs, p.n_lj_pairs, p.n_lj_pairs + p.n_morse_pairs);
+    const int blocks = f.nb[0] * f.nb[1] * f.nb[2];
     // Four points a thread share the x and y separations; grids of so few blocks
     // that this would not fill the GPU once take one (slab of 16 px 10.7 -> 7.5
     // ms, 24 px 13.3 -> 10.3 ms; 64 px 46.2 ms either way, 256 px 478 / 528 ms).
     constexpr int kPoints = kFarP * kFarP * kFarP;
-    if (kPoints / 4 / 128 * (long long)blocks < 3ll * sm_count())
-        far_coef_kernel<1><<<dim3(kPoints / 128, blocks), 128, 0, s>>>(p, f);
-    else
-        far_coef_kernel<4><<<dim3(kPoints / 4 / 128, blocks), 128, 0, s>>>(p, f);
-    far_near_kernel<<<dim3((unsigned)((f.max_strips + 127) / 128), blocks), 128, 0, s>>>(p, f, out);
-    far_interp_kernel<<<dim3((unsigned)f.max_planes, blocks), 256, 0, s>>>(p, f, out, out64);
-    return cudaGetLastError();
+    const bool few = kPoints / 4 / 128 * (long long)blocks < 3ll * sm_count();
+    for (FarViewDF c = f; c.first < blocks; c.first += kFarChunk) {
+        const unsigned n = (unsigned)std::min(kFarChunk, blocks - c.first);
+        far_classify_kernel<<<n, 128, 0, s>>>(c, p.pairs, p.n_lj_pairs, p.n_lj_pairs + p.n_morse_pairs);
+        if (few) far_coef_kernel<1><<<dim3(kPoints / 128, n), 128, 0, s>>>(p, c);
+        else far_coef_kernel<4><<<dim3(kPoints / 4 / 128, n), 128, 0, s>>>(p, c);
+        far_near_kernel<<<dim3((unsigned)((f.max_strips + 127) / 128), n), 128, 0, s>>>(p, c, out);
+        far_interp_kernel<<<dim3((unsigned)f.max_planes, n), 256, 0, s>>>(p, c, out, out64);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_grid_builddf(const ScanParamsDF& p, NodeDF* out, Node64* out64, unsigned* err_word,

@@ -635,8 +635,9 @@ void ensure_far_plan(mafm_scan& s, cudaStream_t st) {
         }
         try {
             s.far_tables.alloc(host.size());
-            s.far_mask.alloc((size_t)blocks * plan.words);
-            s.far_coef.alloc((size_t)blocks * kFarPoints * kFarPoints * kFarPoints);
+            const size_t chunk = (size_t)std::min<long long>(blocks, kFarChunk);
+            s.far_mask.alloc(chunk * plan.words);
+            s.far_coef.alloc(chunk * kFarPoints * kFarPoints * kFarPoints);
         } catch (const Failure&) {   // no room beside the grid: the direct sum needs none
             cudaGetLastError();
             s.far_tables.release();
@@ -657,6 +658,7 @@ void ensure_far_plan(mafm_scan& s, cudaStream_t st) {
             s.far.box[a] = reinterpret_cast<const float2*>(t + at[a][4]);
         }
         s.far.words = plan.words;
+        s.far.first = 0;
         s.far.max_strips = (int)strips;
         s.far.mask = s.far_mask.p;
         s.far.coef = s.far_coef.p;

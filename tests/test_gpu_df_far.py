@@ -65,3 +65,34 @@ def test_far_nodes_keep_their_relative_accuracy(tmp_path, name, attraction):
     size = np.linalg.norm(want[..., :3], axis=-1)
     assert (np.linalg.norm((got - want)[..., :3], axis=-1) / size).max() < 2.0 ** -38
     assert (np.abs(got - want)[..., 3] / np.abs(want[..., 3])).max() < 2.0 ** -38
+
+
+def test_blocks_in_several_launches(tmp_path):
+    """A grid of more blocks than are built at a time: the workspace stays below 67 MB
+    of coefficients and a few of masks and tables, and the nodes are right on both
+    sides of a launch's end."""
+    torch = pytest.importorskip("torch")
+    spec = small_slab(pixels=300, step=0.2, external=False)
+    scan = Scan(_desc(spec, tmp_path), device=0)
+    n, basis, origin = scan.grid_info()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    _abi.check(_abi.lib().mafm_scan_build_grid(scan.handle, _abi.DF, None))
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] - 64 * np.prod(n) < 80e6
+    got, blocks = scan.grid_df()
+    assert np.prod(blocks) > 512
+    # the same terms at every 400th node, the node wrapped into the cell as the build does
+    spec.options["rigidgrid"] = "off"
+    free_desc = _desc(spec, tmp_path)
+    ijk = np.stack(np.unravel_index(np.arange(0, np.prod(n), 401), n), 1)
+    pos = ijk * np.diag(basis) + origin
+    cell, offset = np.array(free_desc.c.cell[:]).reshape(3, 3), np.array(free_desc.c.offset[:])
+    turns = (pos - offset)[:, :2] / np.diag(cell)[:2]
+    inside = (np.abs(turns - np.round(turns)) > 1e-9).all(1)   # either image is right on the border
+    pos[:, :2] -= np.floor(turns) * np.diag(cell)[:2]
+    want = Scan(free_desc, device=0).sample(pos[inside])
+    have = got[tuple(ijk[inside].T)]
+    size = np.linalg.norm(want[:, :3], axis=1)
+    assert inside.mean() > 0.9
+    assert (np.linalg.norm((have - want)[:, :3], axis=1) / size).max() < 1e-8   # positions of 30 A in other roundings
