@@ -145,10 +145,9 @@ bool plan_far_df(const ScanParams& p, const GridView& g, const std::vector<float
 // Simulation::buildTipGridInteractions (simulation.cpp:420-501) in
 // double-float: the rigid grid of geometry p.grid (p.ts_mode 0 or 1: the
 // terms, and the external field) into out, then its FP64 copy (each node's
-// h + l, exact in FP64) into out64 for the FP64 re-relaxation; device error
-// bits (a lookup of the external field) are ORed into *err_word.  far: the plan
-// of the interpolated build, null for every term at every node.
-cudaError_t launch_grid_builddf(const ScanParamsDF& p, NodeDF* out, Node64* out64, unsigned* err_word,
-                                const FarViewDF* far, cudaStream_t s);
+// h + l, exact in FP64) into out64 for the FP64 re-relaxation.  far: the plan of
+// the interpolated build, null for every term at every node.
+cudaError_t launch_grid_builddf(const ScanParamsDF& p, NodeDF* out, Node64* out64, const FarViewDF* far,
+                                cudaStream_t s);
 
 }  // namespace mafm

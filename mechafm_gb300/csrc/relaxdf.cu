@@ -906,13 +906,11 @@ __device__ __forceinline__ void strip_record(const ScanParamsDF& p, int r, D2 tx
 // (ts_mode 1: with the external field).  The x and y separations of a record
 // and their squares are formed once for the strip.
 template <int NB>
-__global__ void __launch_bounds__(128) grid_builddf_kernel(const ScanParamsDF p, NodeDF* out,
-                                                           unsigned* err_word) {
+__global__ void __launch_bounds__(128) grid_builddf_kernel(const ScanParamsDF p, NodeDF* out) {
     const GridViewDF& g = p.grid;
     const int nzs = (g.n[2] + NB - 1) / NB;
     const long long total = (long long)g.n[0] * g.n[1] * nzs;
     const int n_all = p.n_lj_pairs + p.n_morse_pairs;
-    unsigned err = 0;
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
         const int k0 = (int)(idx % nzs) * NB;
@@ -943,7 +941,6 @@ __global__ void __launch_bounds__(128) grid_builddf_kernel(const ScanParamsDF p,
             out[ij * g.n[2] + k0 + m] = NodeDF{F.x, F.y, F.z, E};
         }
     }
-    if (err) atomicOr(err_word, err);
 }
 
 // Each double-float node as FP64: h + l (exact, both parts fit 53 bits).
@@ -1482,8 +1479,8 @@ static cudaError_t launch_far(const ScanParamsDF& p, NodeDF* out, Node64* out64,
     return cudaSuccess;
 }
 
-cudaError_t launch_grid_builddf(const ScanParamsDF& p, NodeDF* out, Node64* out64, unsigned* err_word,
-                                const FarViewDF* far, cudaStream_t s) {
+cudaError_t launch_grid_builddf(const ScanParamsDF& p, NodeDF* out, Node64* out64, const FarViewDF* far,
+                                cudaStream_t s) {
     const long long n = (long long)p.grid.n[0] * p.grid.n[1] * p.grid.n[2];
     if (n <= 0) return cudaSuccess;
     if (far) return launch_far(p, out, out64, *far, s);
@@ -1496,7 +1493,7 @@ cudaError_t launch_grid_builddf(const ScanParamsDF& p, NodeDF* out, Node64* out6
     if (e != cudaSuccess) return e;
     if (per_sm <= 0) per_sm = 1;
     const long long blocks = std::max(1ll, std::min((strips + 127) / 128, (long long)sm_count() * per_sm * 8));
-    grid_builddf_kernel<kNB><<<(unsigned)blocks, 128, 0, s>>>(q, out, err_word);
+    grid_builddf_kernel<kNB><<<(unsigned)blocks, 128, 0, s>>>(q, out);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const long long b64 = std::min((n + 255) / 256, (long long)sm_count() * 32);

@@ -681,8 +681,8 @@ void ensure_grid_df(mafm_scan& s, cudaStream_t st, bool rebuild = false) {
     ScanParams bp = build_grid_params(s);
     bp.grid = s.grid_view;
     const ScanParamsDF q = params_df(bp, s.pairsdf.p, s.df_lj_pairs, s.df_morse_pairs, s.esdf.p, s.griddf.p);
-    cuda_check(launch_grid_builddf(q, s.griddf.p, s.griddf64.p, &s.ctr.p->error_word,
-                                   s.far_used ? &s.far : nullptr, st), "grid build");
+    cuda_check(launch_grid_builddf(q, s.griddf.p, s.griddf64.p, s.far_used ? &s.far : nullptr, st),
+               "grid build");
     s.griddf_built = true;
 }
 
@@ -1016,7 +1016,7 @@ int mafm_run(mafm_scan* scan, const mafm_run_opts* opts, mafm_point* out, mafm_r
             BatchScan b{};
             b.p = build_params(*scan);
             b.out = dout;
-                    b.col_begin = cb;
+            b.col_begin = cb;
             b.col_end = ce;
             b.n_pairs_per_eval = scan->n_pairs_per_eval;
             b.has_coulomb = scan->has_coulomb;
