@@ -166,9 +166,10 @@ struct RunCounters {
 // device counters owned by the caller.
 // launch_relax64: list (may be null) gives the columns, else col_begin,
 // col_begin + 1, ...; n_cols of them.  by_column: the points of column c go to
-// out + (c - col_begin) nz, else those of the i-th to out + i nz.
+// out + (c - col_begin) nz, else those of the i-th to out + i nz.  calm: no height
+// starts within 3.5 A of the atoms, so the columns cost about the same.
 cudaError_t launch_relax64(const ScanParams& p, mafm_point* out, RunCounters* ctr, const int* list,
-                           int col_begin, long long n_cols, int pairs_per_eval, bool by_column,
+                           int col_begin, long long n_cols, int pairs_per_eval, bool by_column, bool calm,
                            cudaStream_t s);
 cudaError_t launch_sample64(const ScanParams& p, int what, const double* pts, int64_t n,
                             double* out, RunCounters* ctr, cudaStream_t s);

@@ -17,6 +17,7 @@
 //   pixel column, z descent    simulation.cpp:93-122, system.cpp:28-51, 139-162
 //   rigid grid build           simulation.cpp:420-501
 #include <algorithm>
+#include <climits>
 
 #include "relax64_dev.cuh"
 
@@ -466,8 +467,8 @@ __global__ void __launch_bounds__(32 * W) relax64_kernel(const __grid_constant__
 
 // One thread a column: the same bits, for so many columns that they fill the GPU by
 // themselves and evaluations of so few terms that the rest of a step, which a quad's
-// lanes repeat, is most of the work (thread_per_column).
-__global__ void __launch_bounds__(128) relax64_thread_kernel(const __grid_constant__ ScanParams p, mafm_point* out,
+// lanes repeat, is most of the work (thread_per_column).  One warp a block.
+__global__ void __launch_bounds__(32) relax64_thread_kernel(const __grid_constant__ ScanParams p, mafm_point* out,
                                                              RunCounters* ctr, const int* list, int col_begin,
                                                              long long n_cols, bool by_column, int smem_cap) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -600,29 +601,38 @@ static cudaError_t launch_relax64_g(const ScanParams& p, mafm_point* out, RunCou
 }
 
 // Whether a thread a column is faster than four lanes a column.  The lanes share the
-// terms but repeat the rest of an evaluation, so the fewer terms, the fewer columns
-// it takes; the in-order sums of Coulomb records leave lanes idle and a field's lookup
-// is not shared, so that such scans change over earlier.  Two heights of a scan, one thread / lanes, ms:
-//   rigid grid  6,400 columns 2.92 / 2.46, 10,000 2.92 / 3.52, 160,000 22.6 / 48.7
-//   field and 16 terms  10,000 9.3 / 7.2, 22,500 11.4 / 18.0
-//   LJ + Coulomb, 4 terms  8,100 5.2 / 4.9, 16,900 5.7 / 7.9; 20 terms  16,900 28.9 /
-//     24.3, 40,000 50.5 / 61.0; 60 terms  40,000 141 / 152, 176,000 473 / 579
-//   LJ  10 terms  16,900 5.4 / 6.1; 20 terms  16,900 12.4 / 11.3, 40,000 22.6 / 26.0;
-//     60 terms  40,000 72 / 66, 176,000 203 / 201
-// (4 LJ terms are an exception between 40,000 and 90,000 columns, 3.6 / 3.1 and 3.9 /
-// 3.4: a few long columns are what lasts.)
-static bool thread_per_column(const ScanParams& p, long long n_cols) {
-    const long long terms = p.ts_mode == 2 ? 0 : p.n_terms_direct;
-    return n_cols >= sm_count() * (45 + (p.has_coulomb || p.ts_mode == 1 ? 4 : 10) * terms);
+// terms and nothing else, so lookups and few terms are in favour of a thread; a
+// thread waits for the slowest of 32 columns at every height, so columns that cost
+// differently are in favour of lanes: close to the atoms, not while the tip starts
+// every height 3.5 A above the topmost one (calm).  Times in ms, thread / lanes, of
+// scans at 0.05 A a pixel whose tip starts at 6 A (cluster) and 10 A (plain grid and
+// field) above the atoms, 0.1 A a height:
+//   rigid grid, calm  6,400 columns x 21 10.1 / 8.5, 8,100 10.1 / 12.4, 90,000 x 41 84 /
+//     180; down to 2 A  8,100 233 / 117, 19,600 254 / 267, 90,000 607 / 874
+//   field and 16 terms, calm  10,000 x 11 17.3 / 13.4, 19,600 21 / 29; down to 2.5 A
+//     19,600 410 / 302, 40,000 643 / 661; 36 terms  40,000 x 26 480 / 504, 90,000 935 /
+//     1122, x 36 2294 / 2305; 64 terms  90,000 x 26 2766 / 2527
+//   4 LJ and Coulomb terms, calm  10,000 x 11 14.5 / 11.6, 19,600 x 21 33 / 40, 90,000 89 /
+//     142; down to 2 A  90,000 328 / 337; LJ alone 209 / 206
+//   10 terms  19,600 x 21 82 / 91, 90,000 210 / 293; down to 2 A  90,000 950 / 780
+//   20 terms  19,600 x 21 295 / 219, 90,000 525 / 588; 60 terms  90,000 x 21 2557 / 2212
+static bool thread_per_column(const ScanParams& p, long long n_cols, bool calm) {
+    const int terms = p.n_terms_direct;
+    int per_sm = INT_MAX;   // columns that an SM needs
+    if (p.ts_mode == 2) per_sm = calm ? 48 : 100;
+    else if (p.ts_mode == 1 && terms <= 16) per_sm = calm ? 110 : 260;
+    else if (p.ts_mode == 1 && terms <= 40) per_sm = 400;
+    else if (p.ts_mode == 0 && calm && terms <= 20) per_sm = terms <= 10 ? 110 : 400;
+    return n_cols >= (long long)sm_count() * per_sm;
 }
 
 static cudaError_t launch_relax64_thread(const ScanParams& p, mafm_point* out, RunCounters* ctr, const int* list,
                                          int col_begin, long long n_cols, bool by_column, cudaStream_t s) {
     int cap = 0, per_sm = 0;
     const size_t smem = smem_bytes64(p, cap);
-    // One warp a block spreads the columns over the SMs (20 terms, 40,000 columns: 59.5
-    // -> 50.5 ms); more where every block's copy of the terms would fill the SM.
-    const int threads = smem <= 8 * 1024 ? 32 : 128;
+    // One warp a block spreads the columns over the SMs (20 terms, 40,000 columns x 2
+    // heights: 59.5 -> 50.5 ms with blocks of 128).
+    constexpr int threads = 32;
     cudaError_t e = cudaFuncSetAttribute(relax64_thread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, relax64_thread_kernel, threads, smem);
@@ -633,20 +643,21 @@ static cudaError_t launch_relax64_thread(const ScanParams& p, mafm_point* out, R
 }
 
 // Lanes per column: the fewest that give every SM four warps (an SM starts an
-// FP64 instruction every 19 cycles and a warp one every 64).  Four lanes cost
-// no more FP64 instructions per column than one, 8 / 16 / 32 lanes 9 / 38 / 95 %
-// more (72 LJ terms), because the in-order sums leave more of them idle.
-// Measured with the divide and square root operators, G = 4 / 8 / 16 / 32: 2,601 columns (graphene, 11 heights) 42.1 /
-// 30.5 / 33.9 / 48.0 ms; 90,000 (cluster, 2 heights) 523 / 647 / 784 / 1071 ms.
-// Four warps per column while there are few columns (and terms to share):
-// cluster, 41 heights, one warp / four warps: 1 column 126 / 78 ms, 301 218 /
-// 152, 1,000 305 / 237; graphene without Coulomb, 11 heights: 576 columns 11.6
-// / 9.9, 961 15.9 / 16.9.
+// FP64 instruction every 19 cycles and a warp one every 64).  More lanes leave more
+// of them idle in the in-order sums.  G = 4 / 8 / 16 / 32: 2,601 columns (graphene, 11
+// heights) 37.4 / 25.4 / 27.6 / 42.1 ms; 22,500 (cluster, 2 heights) 89 / 106 / 130 /
+// 182; 5,041 (cluster, 4 heights) 37.9 / 36.7 / 43.4 / 56.3; 1,296 35.1 / 21.8 / 16.0 /
+// 18.0.
+// Four warps per column while there are few columns: cluster, 41 heights, one warp /
+// four warps: 1 column 163 / 103 ms, 301 190 / 125, 1,000 247 / 200; graphene without
+// Coulomb, 11 heights: 576 columns 12.0 / 10.3, 800 14.5 / 15.5, 961 16.6 / 18.7.  (They
+// are faster for 2 to 15 terms too, 100 columns of 4 atoms 5.1 / 3.3 ms, which the
+// bound of 16 terms leaves out.)
 cudaError_t launch_relax64(const ScanParams& p, mafm_point* out, RunCounters* ctr, const int* list,
-                           int col_begin, long long n_cols, int pairs_per_eval, bool by_column,
+                           int col_begin, long long n_cols, int pairs_per_eval, bool by_column, bool calm,
                            cudaStream_t s) {
     if (n_cols <= 0) return cudaSuccess;
-    if (thread_per_column(p, n_cols))
+    if (thread_per_column(p, n_cols, calm))
         return launch_relax64_thread(p, out, ctr, list, col_begin, n_cols, by_column, s);
     int G = 4;
     while (G < 32 && n_cols * G < 32ll * 4 * sm_count()) G *= 2;

@@ -248,6 +248,7 @@ struct mafm_scan {
     bool order_measured = false;          // order from a relaxation's step counts
     mafm::RunCounters* host_ctr = nullptr;   // pinned
     int n_pairs_per_eval = 0;
+    bool calm = false;                         // every height starts 3.5 A above the topmost atom
     int has_coulomb = 0;
     std::vector<int32_t> atom_type;      // type index of each surface atom (adjoint folding)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -414,6 +415,9 @@ void pack_terms(mafm_scan& s, const mafm_scan_desc& d) {
     s.has_coulomb = n_coul > 0;
     s.P.has_coulomb = s.has_coulomb;
     s.n_pairs_per_eval = d.rigidgrid ? 0 : (int)t64.size() + n_coul;
+    double top = -INFINITY;
+    for (int a = 0; a < d.n_atoms; ++a) top = std::max(top, d.pos[3 * a + 2]);
+    s.calm = d.zhigh - (d.nz - 1) * d.dz - d.tip_dummy_d - top > 3.5;
 }
 
 // ElectrostaticPotentialInteraction ctor (interactions.cpp:53-234) on the GPU.
@@ -990,7 +994,7 @@ int mafm_run(mafm_scan* scan, const mafm_run_opts* opts, mafm_point* out, mafm_r
         cuda_check(cudaEventRecord(scan->ev0, st), "cudaEventRecord");
         if (prec == MAFM_FP64) {
             ScanParams p = build_params(*scan);
-            cuda_check(launch_relax64(p, dout, scan->ctr.p, nullptr, cb, ce - cb, scan->n_pairs_per_eval, true, st),
+            cuda_check(launch_relax64(p, dout, scan->ctr.p, nullptr, cb, ce - cb, scan->n_pairs_per_eval, true, scan->calm, st),
                        "relax64 launch");
         } else if (prec == MAFM_DF) {
             // double-float relaxation, then FP64 for the columns it lists
@@ -1198,7 +1202,7 @@ int mafm_run_columns(mafm_scan* scan, const int32_t* columns, int64_t n, mafm_po
         zero_counters(*scan, st);
         cuda_check(cudaEventRecord(scan->ev0, st), "cudaEventRecord");
         cuda_check(launch_relax64(build_params(*scan), dout, scan->ctr.p, dlist.p, 0, n, scan->n_pairs_per_eval,
-                                  false, st), "FP64 column launch");
+                                  false, scan->calm, st), "FP64 column launch");
         cuda_check(cudaEventRecord(scan->ev1, st), "cudaEventRecord");
         if (staged)
             cuda_check(cudaMemcpyAsync(out, dout, n_pts * sizeof(mafm_point), cudaMemcpyDeviceToHost, st),
