@@ -237,10 +237,12 @@ typedef struct mafm_flex_desc {
 /* The flexible topology of a `flexible on` input (storage owned by `in`). */
 int mafm_input_flex_desc(const mafm_input* in, mafm_flex_desc* out);
 
-/* A device-resident flexible scan: one warp relaxes every atom of a pixel
- * column in FP64, each atom's force summed in the reference's interaction
- * order.  Pair and Coulomb terms only (no rigid grid, no external field:
- * the reference refuses both with flexible molecules, parse.cpp:387-395). */
+/* A device-resident flexible scan: a block of eight warps relaxes every atom of
+ * a pixel column in FP64, each atom's force summed in the reference's
+ * interaction order.  Molecules of more than about 8,000 interactions keep
+ * their forces in device memory during a run (24 bytes each and block).  Pair
+ * and Coulomb terms only (no rigid grid, no external field: the reference
+ * refuses both with flexible molecules, parse.cpp:387-395). */
 typedef struct mafm_flex mafm_flex;
 int mafm_flex_create(int device, const mafm_scan_desc* desc, const mafm_flex_desc* flex,
                      mafm_flex** out);
@@ -283,11 +285,10 @@ int mafm_run(mafm_scan* scan, const mafm_run_opts* opts, mafm_point* out,
 /* Relax chosen pixel columns of a scan in plain FP64: for pixels (i, j)
  * given as columns[m] = i*ny + j, in any order and from anywhere in the scan,
  * out[m*nz + k] receives height k (n*nz records, host or device memory, as
- * for mafm_run).  Every sum is added in the
- * reference's order, so the points are bit-identical to mafm_run's MAFM_FP64
- * points.  The pixel loop of Simulation::run (simulation.cpp:78-122) over a
- * sample of pixels: used to check a fast run against FP64 on pixels spread
- * over the whole scan.  Synchronises the stream. */
+ * for mafm_run).  Every sum is added in the reference's order, so the points are
+ * bit-identical to mafm_run's MAFM_FP64 points.  The pixel loop of
+ * Simulation::run (simulation.cpp:78-122) over a sample of pixels: used to
+ * check a fast run against FP64 on pixels spread over the whole scan.  Synchronises the stream. */
 int mafm_run_columns(mafm_scan* scan, const int32_t* columns, int64_t n, mafm_point* out,
                      mafm_run_stats* stats, void* stream);
 

@@ -325,7 +325,7 @@ __device__ void interp_df_grid(const GridViewDF& g, V3D pos, V3D& f, D& e, int& 
 // are summed), so that the vector arithmetic of the minimiser, which every lane of
 // the group would otherwise repeat, costs a third; with fewer lanes every lane
 // holds all three.  The operations of a component are the same: the same bits.
-// 101 x 101 graphene (G = 4) 107.3 -> 104.7 ms, 40 x 40 (G = 8) 11.8 -> 10.8 ms.
+// 40 x 40 x 21 graphene (G = 8) 11.8 -> 10.8 ms; at G = 4 the runs differ by as much.
 struct QuadDF {
     D c;
 };
@@ -976,8 +976,8 @@ __global__ void nodes_df_to_64_kernel(const NodeDF* in, Node64* out, long long n
 // the records and evaluates all of it.
 //
 // Slab of 9,216 records: 64 x 64 px (157 x 157 x 141 nodes) 270 -> 46 ms, 256 x 256
-// px (541 x 541 x 141) 3198 -> 479 ms; and fewer roundings per node: the relaxed
-// forces' error against FP64 falls from 3e-13 to 1e-14.
+// px (541 x 541 x 141) 3198 -> 481 ms; and fewer roundings per node: the nodes'
+// error against FP64 falls from 1.2e-11 to 5.9e-14 rms (40 x 40 px).
 
 constexpr int kFarP = kFarPoints;
 
@@ -1269,10 +1269,11 @@ constexpr size_t kDfSmem = (size_t)(128 / 32) * 2 * kWarpChunk * sizeof(Node64);
 // Default: one lane per column while the columns fill the resident lanes;
 // fewer columns share out their terms, G = the largest power of two up to 8
 // with G x columns <= 1.25 x the resident lanes.  Measured (MAFM_DF_LANES
-// overrides), G = 1 / 2 / 4 / 8: 401 x 401 cluster (160,801 columns, 58,368
-// resident lanes) 768 / 823 / 935 / 1627 ms; 128 x 128 cluster (16,384
-// columns) 183 / 162 / 142 / 182 ms; 101 x 101 graphene (10,201 columns)
-// 147 / 129 / 111 / 158 ms.
+// overrides), 41 heights, G = 1 / 2 / 4 / 8: 401 x 401 cluster (160,801 columns,
+// 58,368 resident lanes) 589 / 721 / 885 / 1396 ms; 128 x 128 cluster at 0.1 A
+// (16,384) 288 / 271 / 275 / 357; 101 x 101 graphene (10,201) 142 / 115 / 102 / 133;
+// 85 x 85 cluster at 0.2 A (7,225) 160 / 108 / 94 / 103; 60 x 60 graphene 118 / 76 / 52 /
+// 53; 40 x 40 cluster at 0.5 A 157 / 103 / 69 / 60.
 int df_lanes_per_column(long long n_cols, int requested) {
     if (requested == 1 || requested == 2 || requested == 4 || requested == 8) return requested;
     if (const char* e = std::getenv("MAFM_DF_LANES")) {

@@ -157,7 +157,7 @@ class FlexDesc:
 
 
 class FlexScan:
-    """A device-resident flexible scan (mafm_flex): FP64, one warp per column."""
+    """A device-resident flexible scan (mafm_flex): FP64, one block per column."""
 
     def __init__(self, desc: Desc, flex: FlexDesc, device: int = -1):
         h = C.c_void_p()
